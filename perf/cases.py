@@ -176,9 +176,9 @@ def tolerance(case):
     """Four times what 28 cells showed, against exact() and with the sums in another order.  Without a PCG it is
     rounding (4e-15).  With one, a system whose residual passes the threshold by a hair may stop one iteration apart:
     4e-10 in FP64; the mixed form's FP32 correction solves leave 9e-9 wherever they end below the threshold.  A
-    Davidson carries that through its iterations, over its eigenvalues' gaps."""
+    Davidson carries that through its iterations, over its eigenvalues' gaps: 2e-7 where one system stopped apart."""
     if case["do"] == "davidson":
-        return {"rel": 1e-7, "max": 1e-5}
+        return {"rel": 1e-6, "max": 1e-4}
     if case["tr2"] < 0:
         return {"rel": 2e-14, "max": 1e-12}
     return {"rel": 4e-8, "max": 1.2e-6} if case["form"] == "mixed" else {"rel": 2e-9, "max": 3e-7}
