@@ -33,68 +33,6 @@ int fail(int code, const std::string& msg) {
 
 namespace {
 
-// Numbering of the stick pairs (pair 0 is (0,0)).  The plane kernels scatter
-// and gather stick s of a plane from thread s % 256 of the CTA, so the order
-// decides which plane offsets one warp instruction touches.  Pairs are taken
-// in (y, x) order, each time the first one whose two sticks land on shared-
-// memory bank slots not yet used by the current half-warp (8-byte elements,
-// offset mod 16) and quarter-warp (16-byte elements, offset mod 8); when none
-// fits, the next in order.
-std::vector<std::pair<int, int>> stick_pair_order(int N, int prune, const std::map<std::pair<int, int>, int>& pairs) {
-  const int nsp = (int)pairs.size();
-  wb::StickTab shape{};
-  shape.prune = prune;
-  shape.nst = 2 * nsp;
-  const bool fused = wb::fft_fusable(N, shape);
-  std::vector<std::pair<int, int>> rest;
-  for (auto& kv : pairs)
-    if (kv.first.first != 0 || kv.first.second != 0) rest.push_back(kv.first);
-  std::stable_sort(rest.begin(), rest.end(), [](const std::pair<int, int>& a, const std::pair<int, int>& b) {
-    return a.second != b.second ? a.second < b.second : a.first < b.first;
-  });
-  auto slots = [&](int x, int y, int& s16, int& s8) {
-    s16 = wb::fft_plane_offset(N, fused, 8, (x + N) % N, (y + N) % N) % 16;
-    s8 = wb::fft_plane_offset(N, fused, 16, (x + N) % N, (y + N) % N) % 8;
-  };
-  std::vector<std::pair<int, int>> order;
-  order.reserve(nsp);
-  order.push_back({0, 0});
-  unsigned used16 = 0, used8 = 0;
-  {
-    int a16, a8;
-    slots(0, 0, a16, a8);
-    used16 = 1u << a16;
-    used8 = 1u << a8;
-  }
-  std::vector<char> taken(rest.size(), 0);
-  size_t first = 0;
-  for (size_t n = 0; n < rest.size(); ++n) {
-    const int lane = 2 * (int)order.size();
-    if (lane % 16 == 0) used16 = 0;
-    if (lane % 8 == 0) used8 = 0;
-    while (taken[first]) ++first;
-    size_t pick = first;
-    int p16 = 0, p8 = 0, m16 = 0, m8 = 0;
-    for (size_t i = first; i < rest.size(); ++i) {
-      if (taken[i]) continue;
-      int a16, a8, b16, b8;
-      slots(rest[i].first, rest[i].second, a16, a8);
-      slots(-rest[i].first, -rest[i].second, b16, b8);
-      if (i == first) { p16 = a16; p8 = a8; m16 = b16; m8 = b8; }
-      if (a16 != b16 && a8 != b8 && !(used16 >> a16 & 1) && !(used16 >> b16 & 1) && !(used8 >> a8 & 1) &&
-          !(used8 >> b8 & 1)) {
-        pick = i; p16 = a16; p8 = a8; m16 = b16; m8 = b8;
-        break;
-      }
-    }
-    taken[pick] = 1;
-    used16 |= (1u << p16) | (1u << m16);
-    used8 |= (1u << p8) | (1u << m8);
-    order.push_back(rest[pick]);
-  }
-  return order;
-}
-
 template <class T>
 int upload(const T* h, size_t n, DBuf& d);
 
@@ -139,15 +77,13 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
   int mmax = 0;
   for (auto& g : gi) mmax = std::max({mmax, std::abs(g.mx), std::abs(g.my), std::abs(g.mz)});
   const int prune = (!rt && 4 * mmax < N && N % 4 == 0) ? 1 : 0;
-  std::vector<std::pair<int, int>> pair_xy;
-  if (!rt) {
-    pair_xy = stick_pair_order(N, prune, pairs);
-  } else {  // the runtime-size path: pairs in (y, x) order
-    for (auto& kv : pairs) pair_xy.push_back(kv.first);
-    std::stable_sort(pair_xy.begin() + 1, pair_xy.end(), [](const std::pair<int, int>& a, const std::pair<int, int>& b) {
-      return a.second != b.second ? a.second < b.second : a.first < b.first;
-    });
-  }
+  // pair 0 is (0,0), the others in (y, x) order: neighbours in x are neighbours in the stick buffer
+  std::vector<std::pair<int, int>> pair_xy{{0, 0}};
+  for (auto& kv : pairs)
+    if (kv.first != std::make_pair(0, 0)) pair_xy.push_back(kv.first);
+  std::stable_sort(pair_xy.begin() + 1, pair_xy.end(), [](const std::pair<int, int>& a, const std::pair<int, int>& b) {
+    return a.second != b.second ? a.second < b.second : a.first < b.first;
+  });
   for (int p = 1; p < nsp; ++p) pairs[pair_xy[p]] = p;
   std::vector<int> gq(npw), gside(npw);
   int xmax = 0;
@@ -175,51 +111,46 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
     gqz[i] = make_int2(2 * gq[r] + gside[r], gi[r].mz);
   }
   for (int p = 0; p < nsp; ++p) spg[p + 1] += spg[p];
-  const int nst = 2 * nsp;
-  std::vector<int> stpos(nst, -1);
-  if (!rt) {
-    for (int p = 0; p < nsp; ++p) {
-      const int x = pair_xy[p].first, y = pair_xy[p].second;
-      stpos[2 * p] = ((y + N) % N) * N + ((x + N) % N);
-      if (p > 0) stpos[2 * p + 1] = ((-y + N) % N) * N + ((-x + N) % N);
-    }
-  } else {
-    // active columns: every x of a stick or its mirror, x in [-xmax, xmax]
-    const int ncols = 2 * xmax + 1, cs = n2 | 1;
+  const int hs = (nsp + 7) / 8 * 8, nst = 2 * hs;
+  // active plane columns: x in [-xmax, xmax]; pruned transforms read every x in
+  // the outer quarters, so there those columns are the active set
+  c->st.xhi = prune ? N / 4 - 1 : xmax;
+  c->st.ncols = prune ? N / 2 : 2 * xmax + 1;
+  const int ncols = c->st.ncols, nlow = c->st.xhi + 1;
+  std::vector<int> cmap((size_t)n2 * ncols, -1), spos(nst, -1);
+  auto place = [&](int stick, int x, int y) {
+    const int xb = (x + n1) % n1, yb = (y + n2) % n2;
+    const int col = xb < nlow ? xb : xb - (n1 - ncols);
+    cmap[(size_t)yb * ncols + col] = stick;
+    if (rt) spos[stick] = (x + xmax) * (n2 | 1) + yb;
+  };
+  for (int p = 0; p < nsp; ++p) {
+    place(p, pair_xy[p].first, pair_xy[p].second);
+    if (p > 0) place(hs + p, -pair_xy[p].first, -pair_xy[p].second);
+  }
+  if (rt) {
     std::vector<int> colx(ncols);
     for (int cidx = 0; cidx < ncols; ++cidx) colx[cidx] = (cidx - xmax + n1) % n1;
-    auto col_of = [&](int x) { return x + xmax; };
-    for (int p = 0; p < nsp; ++p) {
-      const int x = pair_xy[p].first, y = pair_xy[p].second;
-      stpos[2 * p] = col_of(x) * cs + (y + n2) % n2;
-      if (p > 0) stpos[2 * p + 1] = col_of(-x) * cs + (-y + n2) % n2;
-    }
     c->geo.ncols = ncols;
-    c->geo.cs = cs;
-    if (upload(colx.data(), colx.size(), c->rt_colx)) return fail(WB_ERR_NOMEM, "device allocation failed");
+    c->geo.cs = n2 | 1;
+    if (upload(colx.data(), colx.size(), c->rt_colx) || upload(spos.data(), spos.size(), c->stpos))
+      return fail(WB_ERR_NOMEM, "device allocation failed");
   }
   // device copies
   if (c->gqz.ensure(sizeof(int2) * npw) || c->spg.ensure(sizeof(int) * (nsp + 1)) ||
-      c->stpos.ensure(sizeof(int) * nst) || c->perm.ensure(sizeof(int) * npw))
+      c->cmap.ensure(sizeof(int) * cmap.size()) || c->perm.ensure(sizeof(int) * npw))
     return fail(WB_ERR_NOMEM, "device allocation of stick tables failed");
   WB_CU(cudaMemcpy(c->gqz.p, gqz.data(), sizeof(int2) * npw, cudaMemcpyHostToDevice));
   WB_CU(cudaMemcpy(c->spg.p, spg.data(), sizeof(int) * (nsp + 1), cudaMemcpyHostToDevice));
-  WB_CU(cudaMemcpy(c->stpos.p, stpos.data(), sizeof(int) * nst, cudaMemcpyHostToDevice));
+  WB_CU(cudaMemcpy(c->cmap.p, cmap.data(), sizeof(int) * cmap.size(), cudaMemcpyHostToDevice));
   WB_CU(cudaMemcpy(c->perm.p, perm.data(), sizeof(int) * npw, cudaMemcpyHostToDevice));
   c->st.nsp = nsp;
   c->st.nst = nst;
   c->st.sp_gstart = c->spg.as<int>();
   c->st.g_qz = c->gqz.as<int2>();
-  c->st.st_pos = c->stpos.as<int>();
-  c->st.xhi = xmax;
-  c->st.ncols = 2 * xmax + 1;
+  c->st.hs = hs;
+  c->st.cmap = c->cmap.as<int>();
   c->st.prune = prune;
-  if (c->st.prune) {
-    // pruned transforms read every x in the outer quarters, so those columns
-    // are the active set (they are all zero-filled and transformed)
-    c->st.xhi = N / 4 - 1;
-    c->st.ncols = N / 2;
-  }
   if (rt) {
     c->geo.colx = c->rt_colx.as<int>();
     c->geo.spos = c->stpos.as<int>();
@@ -361,16 +292,9 @@ float time_ms(wb_ctx* c, F fn) {
   return best;
 }
 
-// FP64 form: split-K target of the DMMA bra-ket (1, 2 or 4 CTAs per SM) and
-// the one-pass fused or two-pass plane kernel, timed on this batch's still
-// unused buffers (X zeroed; sticks, part and the active list are rewritten
-// by the batch afterwards).
-// The two-pass plane kernel replaces the one-pass one only when it is clearly
-// faster: at small boxes the two time within noise of each other, and a choice
-// made by noise changed which kernel ran from one context to the next (and with
-// it the rounding of every result).
-constexpr float kPlaneSwitch = 0.9f;
-
+// FP64 form: split-K target of the DMMA bra-ket (1, 2 or 4 CTAs per SM), timed
+// on this batch's still unused buffers (X zeroed; part and the active list are
+// rewritten by the batch afterwards).
 int autotune64(wb_ctx* c, int nsys) {
   if (!c->tune.on || c->tune.done64) return WB_OK;
   c->tune.done64 = 1;
@@ -392,23 +316,14 @@ int autotune64(wb_ctx* c, int nsys) {
     });
     if (ms < best) { best = ms; c->tune.dmma_ctas = ctas; }
   }
-  if (!c->kinetic_only && fft_fusable(c->nr, c->st)) {
-    FftArgs fa = c->fa;
-    const int nit = (nsys + 1) / 2;
-    fa.unfused = 0;
-    const float tf = time_ms(c, [&] { fft_plane_vloc(fa, c->sticks.as<double2>(), nit, c->vs.as<double>()); });
-    fa.unfused = 1;
-    const float tu = time_ms(c, [&] { fft_plane_vloc(fa, c->sticks.as<double2>(), nit, c->vs.as<double>()); });
-    c->tune.unfused64 = tu < kPlaneSwitch * tf ? 1 : 0;
-  }
   WB_CU(cudaGetLastError());
   c->tune.ms += std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return WB_OK;
 }
 
-// Mixed form: split-K target of the tcgen05 bra-ket (1..3 CTAs per SM), systems
-// per CTA of the tcgen05 update (64 or 128) and the FP32 plane kernel variant,
-// on the FP32 buffers before the inner solves use them.
+// Mixed form: split-K target of the tcgen05 bra-ket (1..3 CTAs per SM) and systems
+// per CTA of the tcgen05 update (64 or 128), on the FP32 buffers before the inner
+// solves use them.
 int autotune32(wb_ctx* c, int nsys) {
   if (!c->tune.on || c->tune.done32) return WB_OK;
   c->tune.done32 = 1;
@@ -441,15 +356,6 @@ int autotune32(wb_ctx* c, int nsys) {
       if (ms < best) { best = ms; c->tune.update_nj = nj; }
     }
   }
-  if (!c->kinetic_only && fft_fusable(c->nr, c->st)) {
-    FftArgs32 fa = c->fa32;
-    const int nit = (nsys + 1) / 2;
-    fa.unfused = 0;
-    const float tf = time_ms(c, [&] { fft_plane_vloc32(fa, c->sticks32.as<float2>(), nit, c->vs32.as<float>()); });
-    fa.unfused = 1;
-    const float tu = time_ms(c, [&] { fft_plane_vloc32(fa, c->sticks32.as<float2>(), nit, c->vs32.as<float>()); });
-    c->tune.unfused32 = tu < kPlaneSwitch * tf ? 1 : 0;
-  }
   WB_CU(cudaGetLastError());
   c->tune.ms += std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return WB_OK;
@@ -463,7 +369,6 @@ void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const i
   cudaStream_t s = c->stream;
   FftArgs fa = c->fa;
   fa.dcount = dn;
-  fa.unfused = c->tune.unfused64;
   const double* W = c->W.as<double>();
   int M = c->nproj, nkb = c->nkb;
   const double* Wsub = W;
@@ -582,7 +487,6 @@ void apply_A32(wb_ctx* c, const float2* Pv, float2* Tv, const int* cols, const i
   cudaStream_t s = c->stream;
   FftArgs32 fa = c->fa32;
   fa.dcount = dn;
-  fa.unfused = c->tune.unfused32;
   const float* W = c->W32.as<float>();
   int M = c->nproj, nkb = c->nkb;
   if (c->kinetic_only) {
@@ -1195,11 +1099,27 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
   };
   std::vector<double> g2(npw), sq(npw);
   for (int i = 0; i < npw; ++i) { g2[i] = s->g2kin[perm[i]]; sq[i] = s->sqvc[perm[i]]; }
-  std::vector<double> vsc(c->nnr);
+  std::vector<double> vsc;
   if (!c->rt) {
-    for (int i = 0; i < c->nnr; ++i) vsc[i] = s->vrs[i] / (double)c->nnr;
-    if ((rc = upload(twiddles(N).data(), N, c->tw))) return bail(rc);
+    int A = 1, Bn = 1;  // the plane kernels' step factors
+    fft_split(N, &A, &Bn);
+    const std::vector<double2> t = twiddles(N);
+    std::vector<double2> ts(N);
+    for (int k1 = 0; k1 < A; ++k1)
+      for (int n2 = 0; n2 < Bn; ++n2) ts[k1 * Bn + n2] = t[(k1 * n2) % N];
+    if ((rc = upload(ts.data(), N, c->tw))) return bail(rc);
+    // V(r) / N^3 in the plane kernels' real-space layout, from a copy that goes with this block
+    DBuf raw;
+    if ((rc = upload(s->vrs, (size_t)c->nnr, raw)) || c->vs.ensure(sizeof(double) * (size_t)c->nnr)) {
+      raw.release();
+      return bail(rc ? rc : fail(WB_ERR_NOMEM, "device allocation failed"));
+    }
+    plane_layout(raw.as<double>(), c->vs.as<double>(), N, N, N, A, Bn, (double)c->nnr, c->stream);
+    const cudaError_t ev = cudaStreamSynchronize(c->stream);
+    raw.release();
+    if (ev != cudaSuccess) return bail(fail(WB_ERR_CUDA, std::string("V(r) layout: ") + cudaGetErrorString(ev)));
   } else {
+    vsc.resize(c->nnr);
     // V(r) / N at the digit-reversed positions the runtime transforms leave real space in
     const int nx = s->nr1, ny = s->nr2, nz = s->nr3;
     std::vector<int> rx(nx), ry(ny), rz(nz);
@@ -1220,7 +1140,7 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
       return bail(fail(WB_ERR_UNSUPPORTED, "the x-y plane of this box does not fit in shared memory"));
   }
   if ((rc = upload(g2.data(), npw, c->g2kin)) ||
-      (rc = upload(sq.data(), npw, c->sqvc)) || (rc = upload(vsc.data(), c->nnr, c->vs)) ||
+      (rc = upload(sq.data(), npw, c->sqvc)) || (!vsc.empty() && (rc = upload(vsc.data(), vsc.size(), c->vs))) ||
       (rc = upload(s->et, c->nocc, c->et)) || (rc = upload(s->occupation, c->nocc, c->occ)))
     return bail(rc);
   if ((rc = upload_cols(s->evc, s->npwx, c->nocc, perm, c->evc))) return bail(rc);
@@ -1268,7 +1188,7 @@ int wb_ctx_destroy(wb_ctx* c) {
   if (!c) return WB_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  DBuf* bufs[] = {&c->perm, &c->gqz, &c->spg, &c->stpos, &c->tw, &c->g2kin, &c->sqvc, &c->vs, &c->evc, &c->W,
+  DBuf* bufs[] = {&c->perm, &c->gqz, &c->spg, &c->stpos, &c->cmap, &c->tw, &c->g2kin, &c->sqvc, &c->vs, &c->evc, &c->W,
                   &c->D, &c->eprec, &c->et, &c->occ, &c->evcr, &c->iprec, &c->dvg_in, &c->dng_out, &c->aux, &c->dvbox, &c->B,
                   &c->X, &c->G, &c->T, &c->sticks, &c->sticks2, &c->acc, &c->part, &c->C, &c->rho, &c->conv,
                   &c->act, &c->items, &c->nact, &c->ecol, &c->epcol, &c->unconv, &c->items_pp, &c->items_pk,
@@ -1364,8 +1284,7 @@ int wb_get_tuning(const wb_ctx* c, wb_tuning* out) {
   out->dmma_prefetch = c->tune.dmma_pf;
   out->tc_braket_ctas_per_sm = c->tune.umma_ctas;
   out->tc_update_systems = c->tune.update_nj;
-  out->plane_fused_fp64 = fft_fusable(c->nr, c->st) && !c->tune.unfused64;
-  out->plane_fused_mixed = fft_fusable(c->nr, c->st) && !c->tune.unfused32;
+  out->plane_fused_fp64 = out->plane_fused_mixed = c->rt ? 0 : 1;
   out->tuning_ms = c->tune.ms;
   return WB_OK;
 }

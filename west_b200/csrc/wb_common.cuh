@@ -62,6 +62,16 @@ WB_DEV C ctw(C a, C w) {
   return mkc<C>(fma(a.x, w.x, a.y * w.y), fma(a.y, w.x, -a.x * w.y));
 }
 
+// Asynchronous copy of one complex element (8 or 16 bytes, naturally aligned)
+// from global to shared memory, and the wait for all of a thread's copies.
+template <class C>
+WB_DEV void cp_async_elem(C* smem, const C* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (sizeof(C) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+WB_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 // Work units of a launch: the host count, or, when dn is given (launches
 // replayed from a CUDA graph), the count an earlier kernel left in device
 // memory; PAIRS rounds half of it up (two bands per Gamma FFT).

@@ -63,7 +63,7 @@ struct wb_ctx {
   wb::StickTab st{};
   wb::FftArgs fa{};
   // constant device data
-  DBuf perm, gqz, spg, stpos, tw, g2kin, sqvc, vs, evc, W, D, eprec, et, occ, evcr, iprec;
+  DBuf perm, gqz, spg, stpos, cmap, tw, g2kin, sqvc, vs, evc, W, D, eprec, et, occ, evcr, iprec;
   // per-call workspace
   DBuf dvg_in, dng_out, aux, dvbox, B, X, G, T, sticks, sticks2, acc, part, C, rho, conv, act, items, nact,
       ecol, epcol, unconv, items_pp, items_pk, iota_items, fcoef;
@@ -114,7 +114,7 @@ struct wb_ctx {
   // autotuned launch shapes (set on the first batch of each form, then fixed)
   struct Tune {
     int on = 1, done64 = 0, done32 = 0;
-    int dmma_ctas = 2, dmma_pf = 1, umma_ctas = 2, update_nj = 0, unfused64 = 0, unfused32 = 0;
+    int dmma_ctas = 2, dmma_pf = 1, umma_ctas = 2, update_nj = 0;
     float ms = 0.f;
   } tune;
   cudaEvent_t tev0 = nullptr, tev1 = nullptr;

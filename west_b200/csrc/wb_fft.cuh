@@ -4,17 +4,13 @@
 //   step 1: N2 threads per line, each does an N1-point DFT in registers over
 //           elements N2*n1 + n2, multiplies by W_N^(n2*k1) and writes back to
 //           the same positions (thread-private, no barrier needed);
-//   step 2: N1 threads per line, each reads N2 consecutive results, does an
-//           N2-point DFT in registers and writes element k1 + N1*k2 (natural
-//           order).  Reads and writes of one line overlap, so a barrier
-//           separates them.
-// The small DFTs (2, 3, 4, 5 and composites up to 16) are fully unrolled
-// register code.  Twiddles come from a 2N-entry table in shared memory
-// (computed on the host): entries [0, N) are W_N^j = exp(+2 pi i j / N) in
-// natural order, entries [N, 2N) hold the step-1 factors W_N^(n2 k1) at
-// N + k1 N2 + n2, so the lanes of one step read consecutive entries instead of
-// entries k1 apart (a bank conflict).  DIR = +1 is QE's invfft sign, DIR = -1
-// the fwfft sign.  No normalisation is applied here.
+//   step 2: N1 threads per line, each reads N2 consecutive results and does an
+//           N2-point DFT in registers.
+// The small DFTs (2, 3, 4, 5, 7 and composites up to 16) are fully unrolled
+// register code.  The step-1 factors W_N^(n2 k1) = exp(+2 pi i n2 k1 / N) come
+// from an N-entry table in shared memory at k1 N2 + n2 (computed on the host).
+// DIR = +1 is QE's invfft sign, DIR = -1 the fwfft sign.  No normalisation is
+// applied here.
 #pragma once
 #include "wb_common.cuh"
 
@@ -47,13 +43,25 @@ constexpr double kS52 = 0.58778525229247312917;  // sin(4 pi / 5)
 constexpr double kC71 = 0.62348980185873353053, kC72 = -0.22252093395631440429, kC73 = -0.90096886790241912624;
 constexpr double kS71 = 0.78183148246802980871, kS72 = 0.97492791218182360702, kS73 = 0.43388373911755812048;
 
-template <int R> struct Factor2;  // composite radices R = A * B
+// Composite radices R = A * B of the register DFT.  6, 10, 12, 14 and 15 have
+// coprime factors and run the prime-factor map (no inner twiddles); 8, 9 and 16
+// take theirs from literals.
+template <int R> struct Factor2;
 template <> struct Factor2<6> { static constexpr int A = 3, B = 2; };
 template <> struct Factor2<8> { static constexpr int A = 4, B = 2; };
 template <> struct Factor2<9> { static constexpr int A = 3, B = 3; };
 template <> struct Factor2<10> { static constexpr int A = 5, B = 2; };
 template <> struct Factor2<12> { static constexpr int A = 4, B = 3; };
+template <> struct Factor2<14> { static constexpr int A = 7, B = 2; };
+template <> struct Factor2<15> { static constexpr int A = 5, B = 3; };
 template <> struct Factor2<16> { static constexpr int A = 4, B = 4; };
+constexpr bool pfa_radix(int r) { return r == 6 || r == 10 || r == 12 || r == 14 || r == 15; }
+// the inverse of x modulo m (x, m coprime, small)
+constexpr int inv_mod(int x, int m) {
+  for (int i = 1; i < m; ++i)
+    if ((x * i) % m == 1) return i;
+  return 1;
+}
 
 constexpr double kR2 = 0.70710678118654752440;   // sqrt(1/2)
 
@@ -69,11 +77,34 @@ WB_DEV C tw8(C a, int j) {
   return DIR > 0 ? mkc<C>(-c * s, c * d) : mkc<C>(-c * d, -c * s);
 }
 
-// In-register DFT of size R: v[k] <- sum_n v[n] exp(DIR 2 pi i n k / R).
-// NT is the length of the shared twiddle table twN (R divides NT).  C is
+// cos and sin of 2 pi k / 9 (k = 1, 2, 4) and of 2 pi / 16
+constexpr double kC91 = 0.76604444311897803520, kS91 = 0.64278760968653932632;
+constexpr double kC92 = 0.17364817766693034885, kS92 = 0.98480775301220805937;
+constexpr double kC94 = -0.93969262078590838405, kS94 = 0.34202014332566873304;
+constexpr double kC16 = 0.92387953251128675613, kS16 = 0.38268343236508977173;
+
+// a * exp(DIR 2 pi i j / 9), j = 1, 2, 4
+template <int DIR, class C>
+WB_DEV C tw9(C a, int j) {
+  using T = real_t<C>;
+  const C w = j == 1 ? mkc<C>(T(kC91), T(kS91)) : j == 2 ? mkc<C>(T(kC92), T(kS92)) : mkc<C>(T(kC94), T(kS94));
+  return ctw<DIR>(a, w);
+}
+// a * exp(DIR 2 pi i j / 16), j = 1, 2, 3, 4, 6, 9
+template <int DIR, class C>
+WB_DEV C tw16(C a, int j) {
+  using T = real_t<C>;
+  if (j == 2) return tw8<DIR>(a, 1);
+  if (j == 4) return cmul_i<DIR>(a);
+  if (j == 6) return tw8<DIR>(a, 3);
+  const C w = j == 1 ? mkc<C>(T(kC16), T(kS16)) : j == 3 ? mkc<C>(T(kS16), T(kC16)) : mkc<C>(T(-kC16), T(-kS16));
+  return ctw<DIR>(a, w);
+}
+
+// In-register DFT of size R: v[k] <- sum_n v[n] exp(DIR 2 pi i n k / R).  C is
 // double2 or float2.
-template <int R, int DIR, int NT, class C>
-WB_DEV void rdft(C* v, const C* twN) {
+template <int R, int DIR, class C>
+WB_DEV void rdft(C* v) {
   using T = real_t<C>;
   if constexpr (R == 1) {
     return;
@@ -127,6 +158,26 @@ WB_DEV void rdft(C* v, const C* twN) {
     v[1] = cadd(a1, b1); v[6] = csub(a1, b1);
     v[2] = cadd(a2, b2); v[5] = csub(a2, b2);
     v[3] = cadd(a3, b3); v[4] = csub(a3, b3);
+  } else if constexpr (pfa_radix(R)) {
+    // prime-factor map: input n = B n1 + A n2, output k = B (B^-1 mod A) k1 + A (A^-1 mod B) k2 (mod R)
+    constexpr int A = Factor2<R>::A, B = Factor2<R>::B;
+    constexpr int EA = B * inv_mod(B % A, A), EB = A * inv_mod(A % B, B);
+    C z[B][A];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+#pragma unroll
+      for (int a = 0; a < A; ++a) z[b][a] = v[(B * a + A * b) % R];
+      rdft<A, DIR>(z[b]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+      C t[B];
+#pragma unroll
+      for (int b = 0; b < B; ++b) t[b] = z[b][k1];
+      rdft<B, DIR>(t);
+#pragma unroll
+      for (int k2 = 0; k2 < B; ++k2) v[(EA * k1 + EB * k2) % R] = t[k2];
+    }
   } else {
     constexpr int A = Factor2<R>::A, B = Factor2<R>::B;
     C z[B][A];
@@ -134,12 +185,13 @@ WB_DEV void rdft(C* v, const C* twN) {
     for (int b = 0; b < B; ++b) {
 #pragma unroll
       for (int a = 0; a < A; ++a) z[b][a] = v[B * a + b];
-      rdft<A, DIR, NT>(z[b], twN);
+      rdft<A, DIR>(z[b]);
 #pragma unroll
       for (int k1 = 1; k1 < A; ++k1)
         if (b > 0) {
           if constexpr (R == 8) z[b][k1] = tw8<DIR>(z[b][k1], k1);
-          else z[b][k1] = ctw<DIR>(z[b][k1], twN[((b * k1) * (NT / R)) % NT]);
+          else if constexpr (R == 9) z[b][k1] = tw9<DIR>(z[b][k1], b * k1);
+          else z[b][k1] = tw16<DIR>(z[b][k1], b * k1);
         }
     }
 #pragma unroll
@@ -147,7 +199,7 @@ WB_DEV void rdft(C* v, const C* twN) {
       C t[B];
 #pragma unroll
       for (int b = 0; b < B; ++b) t[b] = z[b][k1];
-      rdft<B, DIR, NT>(t, twN);
+      rdft<B, DIR>(t);
 #pragma unroll
       for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = t[k2];
     }
@@ -184,119 +236,52 @@ struct Prune {
   WB_DEV static constexpr bool out_live(int k2) { return k2 < N2 / 4 || k2 >= N2 - N2 / 4; }
 };
 
-// Batched line FFTs in shared memory.  Line l starts at data + loff(l).
-// Elements of a line are either padded-contiguous (PADDED, LinePad layout,
-// element stride 1) or strided by es with no padding (columns of a plane,
-// where consecutive threads take consecutive lines).  LINE_FAST puts
-// consecutive threads on consecutive lines.  The two steps are separate so a
-// kernel can fuse pointwise work between them; fft_lines runs both.  All
-// functions must be called by all NT threads of the block.
-template <int N, int DIR, int NT, bool LINE_FAST, bool PADDED, int PRUNE = PRUNE_NONE, class Off, class C>
-WB_DEV void fft_step1(C* data, Off loff, int es, int nlines, const C* twN) {
+// Batched line FFTs in shared memory (the z passes).  Line l starts at
+// data + l * stride, its elements in the LinePad layout.  Step 1 gives
+// consecutive threads consecutive n2 of a line, step 2 consecutive k1.  Both
+// must be called by all NT threads of the block.
+template <int N, int DIR, int NT, int PRUNE = PRUNE_NONE, class C>
+WB_DEV void fft_lines(C* data, int stride, int nlines, const C* twN) {
   using LP = LinePad<N>;
   using PR = Prune<N>;
   constexpr bool PIN = (PRUNE == PRUNE_IN) && PR::IN_OK;
-  constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2;
-  const int tid = threadIdx.x;
-  const int items1 = nlines * N2;
-  for (int it = tid; it < items1; it += NT) {
-    int line, n2;
-    if (LINE_FAST) { line = it % nlines; n2 = it / nlines; }
-    else { line = it / N2; n2 = it % N2; }
-    C* p = data + loff(line);
-    C v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1)
-      v[n1] = (PIN && !PR::in_live(n1)) ? mkc<C>(0, 0)
-                                        : p[PADDED ? LP::off_blk(n1, n2) : (N2 * n1 + n2) * es];
-    rdft<N1, DIR, N>(v, twN);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) v[k1] = ctw<DIR>(v[k1], twN[N + k1 * N2 + n2]);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) p[PADDED ? LP::off_blk(k1, n2) : (N2 * k1 + n2) * es] = v[k1];
-  }
-}
-
-template <int N, int DIR, int NT, bool LINE_FAST, bool PADDED, int PRUNE = PRUNE_NONE, class Off, class C>
-WB_DEV void fft_step2(C* data, Off loff, int es, int nlines, const C* twN) {
-  using LP = LinePad<N>;
-  using PR = Prune<N>;
   constexpr bool POUT = (PRUNE == PRUNE_OUT) && PR::OUT_OK;
   constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2;
   const int tid = threadIdx.x;
+  for (int it = tid; it < nlines * N2; it += NT) {
+    const int line = it / N2, n2 = it % N2;
+    C* p = data + line * stride;
+    C v[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1)
+      v[n1] = (PIN && !PR::in_live(n1)) ? mkc<C>(0, 0) : p[LP::off_blk(n1, n2)];
+    rdft<N1, DIR>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) v[k1] = ctw<DIR>(v[k1], twN[k1 * N2 + n2]);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) p[LP::off_blk(k1, n2)] = v[k1];
+  }
+  __syncthreads();
   constexpr int LPC = NT / N1;
   const int nchunks = (nlines + LPC - 1) / LPC;
   for (int c = 0; c < nchunks; ++c) {
-    int line, k1;
-    if (LINE_FAST) { line = c * LPC + tid % LPC; k1 = tid / LPC; }
-    else { line = c * LPC + tid / N1; k1 = tid % N1; }
+    const int line = c * LPC + tid / N1, k1 = tid % N1;
     const bool act = (tid < LPC * N1) && (line < nlines);
     C v[N2];
-    C* p = data + (act ? loff(line) : 0);
+    C* p = data + (act ? line * stride : 0);
     if (act) {
 #pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[PADDED ? LP::off_blk(k1, n2) : (N2 * k1 + n2) * es];
-      rdft<N2, DIR, N>(v, twN);
+      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[LP::off_blk(k1, n2)];
+      rdft<N2, DIR>(v);
     }
     __syncthreads();
     if (act) {
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2)
-        if (!POUT || PR::out_live(k2)) p[PADDED ? LP::off(k1 + N1 * k2) : (k1 + N1 * k2) * es] = v[k2];
+        if (!POUT || PR::out_live(k2)) p[LP::off(k1 + N1 * k2)] = v[k2];
     }
   }
   __syncthreads();
 }
-
-template <int N, int DIR, int NT, bool LINE_FAST, bool PADDED, int PRUNE = PRUNE_NONE, class Off, class C>
-WB_DEV void fft_lines(C* data, Off loff, int es, int nlines, const C* twN) {
-  fft_step1<N, DIR, NT, LINE_FAST, PADDED, PRUNE>(data, loff, es, nlines, twN);
-  __syncthreads();
-  fft_step2<N, DIR, NT, LINE_FAST, PADDED, PRUNE>(data, loff, es, nlines, twN);
-}
-
-struct OffLinear {
-  int stride;
-  WB_DEV int operator()(int l) const { return l * stride; }
-};
-// Active columns of a padded plane: x in [0, xhi] and [N - (ncols - nlow), N).
-template <int N>
-struct OffCols {
-  int nlow, ncols;
-  WB_DEV int operator()(int l) const { return LinePad<N>::off(l < nlow ? l : N - ncols + l); }
-};
-
-// Plane of N x N complex values: rows are padded lines (LinePad), row stride RS.
-template <int N>
-struct Plane {
-  static constexpr int RS = LinePad<N>::LEN;
-  static constexpr int SIZE = N * RS;
-  WB_HD static int row(int y) { return y * RS; }
-  WB_HD static int at(int x, int y) { return y * RS + LinePad<N>::off(x); }
-  // plane offset of the e-th element in row-major (y*N + x) order
-  WB_HD static int at_lin(int e) { return at(e % N, e / N); }
-};
-
-// Plane of the fused local-potential kernel.  For N = 8 x 8 with 8-byte
-// elements (FP32 complex) every group of 8 rows is shifted by GP = 8 more
-// elements.  A half-warp of 8-byte accesses covers 16 bank slots (offset mod
-// 16); the row stride 72 puts rows y and y+1 eight slots apart, and the group
-// shift does the same for rows y and y+8, so the column passes can give each
-// half-warp one aligned block of 8 columns in two rows 1 or 8 apart without a
-// conflict (16-byte elements are served per quarter-warp, one row, and need
-// no shift).
-template <int N, class C>
-struct FPlane {
-  static constexpr int R = FftSplit<N>::N1;
-  static constexpr int RS = LinePad<N>::LEN;
-  static constexpr int GP = (sizeof(C) == 8 && R == 8 && FftSplit<N>::N2 == 8) ? 8 : 0;
-  static constexpr int GS = R * RS + GP;  // stride between groups of R rows
-  static constexpr int SIZE = N * RS + (N / R) * GP;
-  // row y = R * a + b with b in [0, R)
-  WB_HD static int row2(int a, int b) { return a * GS + b * RS; }
-  WB_HD static int row(int y) { return row2(y / R, y % R); }
-  WB_HD static int at(int x, int y) { return row(y) + LinePad<N>::off(x); }
-  WB_HD static int at_lin(int e) { return at(e % N, e / N); }
-};
 
 }  // namespace wb

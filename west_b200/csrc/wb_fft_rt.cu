@@ -83,7 +83,7 @@ WB_DEV void rt_bfly(C* p, int es, int base, int m, int j, int ts, const C* tw) {
 #pragma unroll
     for (int q = 1; q < R; ++q) v[q] = ctw<DIR>(v[q], tw[q * j * ts]);
   }
-  rdft<R, DIR, 8>(v, tw);  // R <= 8: exact constants, no table
+  rdft<R, DIR>(v);
   if (DIF && j) {
 #pragma unroll
     for (int q = 1; q < R; ++q) v[q] = ctw<DIR>(v[q], tw[q * j * ts]);
@@ -135,8 +135,10 @@ WB_DEV C* rt_smem() {
 }
 
 // ---------------------------------------------------------------------------
-// z passes
+// z passes: line side * kRtZsg + i of the work area is that stick of pair q0 + i
 // ---------------------------------------------------------------------------
+WB_DEV int rt_line(int l) { return (l & 1) * kRtZsg + (l >> 1); }
+
 template <class C>
 __global__ void __launch_bounds__(kRtZnt) k_zinv_rt(const C* __restrict__ src, long ld,
                                                     const int2* __restrict__ items, StickTab st, RtGeo g,
@@ -166,18 +168,17 @@ __global__ void __launch_bounds__(kRtZnt) k_zinv_rt(const C* __restrict__ src, l
       if (z != 0) { zb[(z + N) % N] = pos; zb[(N - z) % N] = neg; }
       else zb[0] = neg;  // G = 0: the -G store wins, as in the reference loop
     } else {
-      const int l = qz.x - 2 * q0;
+      const int l = rt_line(qz.x - 2 * q0);  // its mirror is l ^ kRtZsg
       zb[l * LS + (z + N) % N] = pos;
-      zb[(l ^ 1) * LS + (N - z) % N] = neg;
+      zb[(l ^ kRtZsg) * LS + (N - z) % N] = neg;
     }
   }
   __syncthreads();
-  rt_lines<+1, true>(zb, RtOff{LS}, 1, 2 * nq, g.pz, tw);
-  const int ns = 2 * nq;
-  C* o = out + (long)item * N * st.nst + 2 * q0;
-  for (int e = threadIdx.x; e < ns * N; e += kRtZnt) {
-    const int s = e % ns, pz = e / ns;
-    o[(long)pz * st.nst + s] = zb[s * LS + pz];
+  rt_lines<+1, true>(zb, RtOff{LS}, 1, 2 * kRtZsg, g.pz, tw);
+  C* o = out + (long)item * N * st.nst + q0;
+  for (int e = threadIdx.x; e < 2 * kRtZsg * N; e += kRtZnt) {
+    const int l = e % (2 * kRtZsg), pz = e / (2 * kRtZsg);
+    if (l % kRtZsg < nq) o[(long)pz * st.nst + (l / kRtZsg) * st.hs + l % kRtZsg] = zb[l * LS + pz];
   }
 }
 
@@ -192,15 +193,15 @@ __global__ void __launch_bounds__(kRtZnt) k_zfwd_rt(const C* __restrict__ sticks
   const C* twg = rt_table<C>(g.twz, g.twz32);
   const int q0 = blockIdx.x * kRtZsg, item = blockIdx.y;
   const int nq = min(kRtZsg, st.nsp - q0);
-  const int ns = 2 * nq;
-  const C* s0 = sticks + (long)item * N * st.nst + 2 * q0;
-  for (int i = threadIdx.x; i < N; i += kRtZnt) tw[i] = twg[i];
-  for (int e = threadIdx.x; e < ns * N; e += kRtZnt) {
-    const int s = e % ns, pz = e / ns;
-    zb[s * LS + pz] = s0[(long)pz * st.nst + s];
+  const C* s0 = sticks + (long)item * N * st.nst + q0;
+  for (int e = threadIdx.x; e < 2 * kRtZsg * N; e += kRtZnt) {
+    const int l = e % (2 * kRtZsg), pz = e / (2 * kRtZsg);
+    if (l % kRtZsg < nq) cp_async_elem(zb + l * LS + pz, s0 + (long)pz * st.nst + (l / kRtZsg) * st.hs + l % kRtZsg);
   }
+  for (int i = threadIdx.x; i < N; i += kRtZnt) tw[i] = twg[i];
+  cp_async_wait_all();
   __syncthreads();
-  rt_lines<-1, false>(zb, RtOff{LS}, 1, ns, g.pz, tw);
+  rt_lines<-1, false>(zb, RtOff{LS}, 1, 2 * kRtZsg, g.pz, tw);
   const int2 it = items[item];
   const int g0 = st.sp_gstart[q0], g1 = st.sp_gstart[q0 + nq];
   for (int gi = g0 + threadIdx.x; gi < g1; gi += kRtZnt) {
@@ -212,9 +213,9 @@ __global__ void __launch_bounds__(kRtZnt) k_zfwd_rt(const C* __restrict__ sticks
       ap = zb[(z + N) % N];
       am = zb[(N - z) % N];
     } else {
-      const int l = qz.x - 2 * q0;
+      const int l = rt_line(qz.x - 2 * q0);
       ap = zb[l * LS + (z + N) % N];
-      am = zb[(l ^ 1) * LS + (N - z) % N];
+      am = zb[(l ^ kRtZsg) * LS + (N - z) % N];
     }
     const C fp = mkc<C>(T(0.5) * (ap.x + am.x), T(0.5) * (ap.y + am.y));
     const C fm = mkc<C>(T(0.5) * (ap.x - am.x), T(0.5) * (ap.y - am.y));

@@ -9,10 +9,11 @@ namespace wb {
 // Stick decomposition of the Gamma half sphere (built on the host from nl).
 struct StickTab {
   int nsp;               // stick pairs; pair 0 is the (0,0) stick
-  int nst;               // sticks in the buffer = 2 * nsp (stick 1 is a dummy)
+  int nst;               // sticks in the buffer = 2 * hs
+  int hs;                // stick side * hs + q is side 0 or 1 of pair q (hs >= nsp)
   const int* sp_gstart;  // [nsp + 1] first internal G index of each pair
   const int2* g_qz;      // [npw] (2 * pair + side, signed z) of each internal G
-  const int* st_pos;     // [nst] plane offset y*N + x of each stick, -1 = dummy
+  const int* cmap;       // [y][active column] stick at (x, y), -1 = none
   int xhi;               // active plane columns: x in [0, xhi] and [N - (ncols - xhi - 1), N)
   int ncols;
   int prune;             // 1 if every |Miller index| < N/4 (sphere inside the outer quarters)
@@ -54,10 +55,9 @@ size_t rt_plane_smem(const RtGeo& g, int elem_bytes, int* rows_per_chunk);
 struct FftArgs {
   int n;                 // box edge (0 when the runtime-size path runs)
   StickTab st;
-  const double2* tw;     // [n] exp(+2 pi i j / n)
+  const double2* tw;     // [n] step factors W_n^(k1 n2) at k1 N2 + n2 (wb_fft.cuh)
   cudaStream_t stream;
   const int* dcount = nullptr;
-  int unfused = 0;       // 1: the two-pass plane kernel even where the fused one applies
   const RtGeo* rt = nullptr;  // runtime-size path when set
 };
 
@@ -68,7 +68,6 @@ struct FftArgs32 {
   const float2* tw;
   cudaStream_t stream;
   const int* dcount = nullptr;
-  int unfused = 0;
   const RtGeo* rt = nullptr;
 };
 
@@ -91,12 +90,12 @@ void rt_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evcr
 void rt_setup(const RtGeo& g);
 
 bool fft_supported(int n);
-// the fused one-pass plane kernel applies to this box and stick table
-bool fft_fusable(int n, const StickTab& st);
-// offset of plane element (x, y) in the shared-memory plane of the x-y pass
-// kernels: the fused local-potential layout (fused) or the padded-row one,
-// for elem_bytes 8 (FP32 complex) or 16 (FP64 complex)
-int fft_plane_offset(int n, bool fused, int elem_bytes, int x, int y);
+// the split n = a * b of a compiled edge's line transforms: the plane kernels
+// keep y = k1 + a k2 of real space at row b k1 + k2 (0, 0 for other edges)
+void fft_split(int n, int* a, int* b);
+// out[z][x][ys] = in[z][y][x] / div, ys = b (y mod a) + y / a: the plane
+// kernels' real-space layout (wb_plane.cuh)
+void plane_layout(const double* in, double* out, int nx, int ny, int nz, int a, int b, double div, cudaStream_t s);
 
 // Davidson restart hand-off in WEST's layout (Wstat/davidson_restart.f90):
 // <dir>/summary.json (dav_iter, notcnv, nbase, conv, ev, ew), <dir>/hr_vr.dat

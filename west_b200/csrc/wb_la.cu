@@ -355,6 +355,20 @@ void kinetic_hpsi(const double2* P, double2* T, const double* g2kin, const doubl
   k_kinetic_hpsi<<<dim3((npw + 255) / 256, ncol), 256, 0, s>>>(P, T, g2kin, ecol, cols, dn, npw, ld);
 }
 
+__global__ void k_plane_layout(const double* __restrict__ in, double* __restrict__ out, int nx, int ny, long n, int a,
+                               int b, double div) {
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
+    const int ys = (int)(e % ny), x = (int)(e / ny % nx);
+    const long z = e / ((long)nx * ny);
+    const int y = ys / b + a * (ys % b);
+    out[e] = in[(z * ny + y) * nx + x] / div;
+  }
+}
+void plane_layout(const double* in, double* out, int nx, int ny, int nz, int a, int b, double div, cudaStream_t s) {
+  const long n = (long)nx * ny * nz;
+  k_plane_layout<<<(int)std::min<long>((n + 255) / 256, 4096), 256, 0, s>>>(in, out, nx, ny, n, a, b, div);
+}
+
 // eprec_v = 1.35 sum_G |psi_v(G)|^2 g2kin(G)       (set_eprec.f90:40-53)
 __global__ void __launch_bounds__(256) k_set_eprec(const double2* __restrict__ evc, const double* __restrict__ g2kin,
                                                    int npw, double* __restrict__ eprec) {
