@@ -245,7 +245,6 @@ int ensure_workspace(wb_ctx* c, int mb, long ld_in, long ld_out) {
   const size_t stk1 = sizeof(double2) * (size_t)c->nz * c->st.nst;
   const size_t mp = (mb + 1) / 2;
   const size_t nitems = std::max<size_t>({(nsys + 1) / 2, (size_t)mb * c->npv, mp, (size_t)c->npv});
-  const int nsplit = gemm_tn_splits(c->nproj, (int)nsys, 2 * c->npw, 4);  // the tuner's largest target
   bool bad = false;
   bad |= c->dvg_in.ensure(sizeof(double2) * ld_in * mb + 16) != 0;
   bad |= c->dng_out.ensure(sizeof(double2) * ld_out * mb + 16) != 0;
@@ -255,8 +254,9 @@ int ensure_workspace(wb_ctx* c, int mb, long ld_in, long ld_out) {
   bad |= c->sticks.ensure(stk1 * nitems) != 0;
   bad |= c->sticks2.ensure(stk1 * mp) != 0;
   bad |= c->acc.ensure(sizeof(double2) * (size_t)c->nnr * mp) != 0;
-  bad |= c->part.ensure(sizeof(double) * std::max((size_t)nsplit * nsys * c->nproj,
-                                                   gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw, 4))) != 0;
+  // all projectors or the bands alone, up to the tuner's largest target
+  bad |= c->part.ensure(sizeof(double) * std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw, 4),
+                                                   gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw, 4))) != 0;
   bad |= c->C.ensure(sizeof(double) * nsys * c->nproj) != 0;
   bad |= c->rho.ensure(sizeof(double) * nsys) != 0;
   bad |= c->conv.ensure(nsys + 16) != 0;
@@ -309,10 +309,10 @@ int autotune64(wb_ctx* c, int nsys) {
   cg_compact(c->conv.as<unsigned char>(), nsys, c->act.as<int>(), c->items.as<int2>(), c->nact.as<int>(), nullptr, s);
   float best = 3.4e38f;
   for (int ctas : {1, 2, 4}) {
-    const int ns = gemm_tn_splits(M, nsys, K, ctas);
+    const int ns = gemm_tn_plan(M, nsys, K, ctas);
     const float ms = time_ms(c, [&] {
       gemm_tn(W, K, M, (const double*)c->X.p, 2 * ld, c->act.as<int>(), nsys, K, ns, c->part.as<double>(), s,
-              nullptr, ctas, c->tune.dmma_pf);
+              nullptr, ctas);
     });
     if (ms < best) { best = ms; c->tune.dmma_ctas = ctas; }
   }
@@ -361,9 +361,25 @@ int autotune32(wb_ctx* c, int nsys) {
   return WB_OK;
 }
 
+// A branch of the pass being captured on the context's second stream, and its
+// end.  It pays while a pass is launch and chain latency (one perturbation at
+// 64^3: 5.0 -> 4.7 ms a call, at 24^3 0.86 -> 0.75); with hundreds of systems
+// every kernel fills the GPU and the two branches only share its L2 (108^3, 512
+// systems: 276 against 284 ms).
+bool forked(const wb_ctx* c, int nmax) { return (double)nmax * c->npw <= 8e6; }
+cudaStream_t fork_side(wb_ctx* c) {
+  cudaEventRecord(c->side_ev[0], c->stream);
+  cudaStreamWaitEvent(c->side, c->side_ev[0], 0);
+  return c->side;
+}
+void join_side(wb_ctx* c) {
+  cudaEventRecord(c->side_ev[1], c->side);
+  cudaStreamWaitEvent(c->stream, c->side_ev[1], 0);
+}
+
 // dn: device count of the listed columns (graph replays; n is then the maximum).
-void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const int2* items, int n, int nsys,
-             int nsplit, const int* dn = nullptr) {
+void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const int2* items, int n,
+             const int* dn = nullptr) {
   const long ld = c->npw;
   const int K = 2 * c->npw;
   cudaStream_t s = c->stream;
@@ -373,11 +389,28 @@ void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const i
   int M = c->nproj, nkb = c->nkb;
   const double* Wsub = W;
   if (c->kinetic_only) {
-    Stage g(c, WB_STAGE_VLOC_ZFWD, 1, n);
-    kinetic_hpsi(Xv, Tv, c->g2kin.as<double>(), c->ecol.as<double>(), cols, n, c->npw, ld, s, dn);
     Wsub = W + (size_t)c->nkb * K;  // alpha Pv only
     M = c->nocc;
     nkb = 0;
+  }
+  // In a captured pass the bra-ket and its reduction, which need X alone, are a
+  // second branch beside the local potential.
+  const int nsplit = gemm_tn_plan(M, n, K, c->tune.dmma_ctas);
+  const bool side = dn && forked(c, n);
+  const cudaStream_t sb = side ? fork_side(c) : s;
+  {
+    Stage g(c, WB_STAGE_GEMM_TN, 1, n);
+    gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, nsplit, c->part.as<double>(), sb, dn,
+            c->tune.dmma_ctas);
+  }
+  {
+    Stage g(c, WB_STAGE_GEMM_REDUCE, 1, n);
+    gamma_reduce(c->part.as<double>(), nsplit, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(),
+                 nkb, c->alpha, c->C.as<double>(), sb, dn, K, c->tune.dmma_ctas);
+  }
+  if (c->kinetic_only) {
+    Stage g(c, WB_STAGE_VLOC_ZFWD, 1, n);
+    kinetic_hpsi(Xv, Tv, c->g2kin.as<double>(), c->ecol.as<double>(), cols, n, c->npw, ld, s, dn);
   } else {
     const int nit = (n + 1) / 2;
     {
@@ -395,21 +428,11 @@ void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const i
     }
     c->stats.fft_boxes += 2 * nit;
   }
-  {
-    Stage g(c, WB_STAGE_GEMM_TN, 1, n);
-    gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, nsplit, c->part.as<double>(), s, dn,
-            c->tune.dmma_ctas, c->tune.dmma_pf);
-  }
-  {
-    Stage g(c, WB_STAGE_GEMM_REDUCE, 1, n);
-    gamma_reduce(c->part.as<double>(), nsplit, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(),
-                 nkb, c->alpha, c->C.as<double>(), s, dn, K, c->tune.dmma_ctas);
-  }
+  if (side) join_side(c);
   {
     Stage g(c, WB_STAGE_GEMM_NN, 1, n);
     gemm_nn(Wsub, K, M, c->C.as<double>(), (double*)Tv, 2 * ld, cols, n, K, 1.0, s, dn);
   }
-  (void)nsys;
 }
 
 // ---------------------------------------------------------------------------
@@ -490,11 +513,28 @@ void apply_A32(wb_ctx* c, const float2* Pv, float2* Tv, const int* cols, const i
   const float* W = c->W32.as<float>();
   int M = c->nproj, nkb = c->nkb;
   if (c->kinetic_only) {
-    Stage g(c, WB_STAGE_VLOC_ZFWD, 1, n);
-    kinetic_hpsi32(Pv, Tv, c->g2kin32.as<float>(), c->ecol32.as<float>(), cols, n, c->npw, ld, s, dn);
     W += (size_t)c->nkb * K;
     M = c->nocc;
     nkb = 0;
+  }
+  const bool side = dn && forked(c, n);  // as in apply_A
+  const cudaStream_t sb = side ? fork_side(c) : s;
+  {
+    Stage g(c, WB_STAGE_GEMM_TN, 1, n);
+    if (c->umma)
+      nsplit = umma_braket(c->umma_braket_w.p, M, (const float*)Pv, 2 * ld, cols, n, K, c->part32.as<float>(),
+                           c->umma_err.as<int>(), sb, dn, c->tune.umma_ctas);
+    else
+      gemm_tn32(W, K, M, (const float*)Pv, 2 * ld, cols, n, K, nsplit, c->part32.as<float>(), sb, dn);
+  }
+  {
+    Stage g(c, WB_STAGE_GEMM_REDUCE, 1, n);
+    gamma_reduce32(c->part32.as<float>(), nsplit, M, n, W, K, (const float*)Pv, 2 * ld, cols, c->D32.as<float>(), nkb,
+                   (float)c->alpha, c->C32.as<float>(), sb, dn, K, c->umma ? c->tune.umma_ctas : 0);
+  }
+  if (c->kinetic_only) {
+    Stage g(c, WB_STAGE_VLOC_ZFWD, 1, n);
+    kinetic_hpsi32(Pv, Tv, c->g2kin32.as<float>(), c->ecol32.as<float>(), cols, n, c->npw, ld, s, dn);
   } else {
     const int nit = (n + 1) / 2;
     {
@@ -512,19 +552,7 @@ void apply_A32(wb_ctx* c, const float2* Pv, float2* Tv, const int* cols, const i
     }
     c->stats.fft_boxes += 2 * nit;
   }
-  {
-    Stage g(c, WB_STAGE_GEMM_TN, 1, n);
-    if (c->umma)
-      nsplit = umma_braket(c->umma_braket_w.p, M, (const float*)Pv, 2 * ld, cols, n, K, c->part32.as<float>(),
-                           c->umma_err.as<int>(), s, dn, c->tune.umma_ctas);
-    else
-      gemm_tn32(W, K, M, (const float*)Pv, 2 * ld, cols, n, K, nsplit, c->part32.as<float>(), s, dn);
-  }
-  {
-    Stage g(c, WB_STAGE_GEMM_REDUCE, 1, n);
-    gamma_reduce32(c->part32.as<float>(), nsplit, M, n, W, K, (const float*)Pv, 2 * ld, cols, c->D32.as<float>(), nkb,
-                   (float)c->alpha, c->C32.as<float>(), s, dn, K, c->umma ? c->tune.umma_ctas : 0);
-  }
+  if (side) join_side(c);
   {
     Stage g(c, WB_STAGE_GEMM_NN, 1, n);
     if (c->umma)
@@ -551,7 +579,10 @@ bool graph_mode(const wb_ctx* c) { return c->use_graphs && c->prof == 0; }
 // up to kMinBucketItems << k band-pair items } -> k_loop_ctl }.  Each branch
 // launches the same kernels as the eager loop with grids for its bucket; the
 // CTAs beyond the device count return at once, so at most half a grid idles.
-constexpr int kMinBucketItems = 16;
+// A workspace of one bucket needs no SWITCH: WHILE { one PCG pass }, whose step
+// kernel counts the pass and sets the condition (two launches and a conditional
+// node less of about ten per pass, where a pass takes 50 us).
+constexpr int kMinBucketItems = 32;
 
 template <class Pass>
 int capture_loop(wb_ctx* c, wb_ctx::LoopCache& cache, std::vector<const void*> key, double tr2, int cap,
@@ -584,43 +615,44 @@ int capture_loop(wb_ctx* c, wb_ctx::LoopCache& cache, std::vector<const void*> k
     wp.conditional.size = 1;
     e = cudaGraphAddNode(&wnode, lg.graph, nullptr, 0, &wp);
   }
-  if (e == cudaSuccess) {
-    body = wp.conditional.phGraph_out[0];
-    e = cudaGraphConditionalHandleCreate(&hs, body, 0, 0);
+  if (e == cudaSuccess) body = wp.conditional.phGraph_out[0];
+  CgLoop loop{};
+  loop.st = st;
+  loop.inner = shared_budget ? 1 : 0;
+  auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* after, size_t n_after, auto enqueue) {
+    cudaError_t r = cudaStreamBeginCaptureToGraph(s, into, after, nullptr, n_after, cudaStreamCaptureModeThreadLocal);
+    if (r != cudaSuccess) return r;
+    enqueue();
+    cudaGraph_t g = nullptr;
+    return cudaStreamEndCapture(s, &g);
+  };
+  if (nb == 1) {
+    loop.cond = hw;
+    loop.ctl = 1;
+    if (e == cudaSuccess) e = capture(body, nullptr, 0, [&] { pass(cap, loop); });
+  } else {
+    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hs, body, 0, 0);
+    // 1. the bucket of this pass
+    if (e == cudaSuccess)
+      e = capture(body, nullptr, 0, [&] { loop_bucket(hs, dn, st, kMinBucketItems, nb, s); });
+    size_t nn = 1;
+    if (e == cudaSuccess) e = cudaGraphGetNodes(body, &bnode, &nn);
+    // 2. SWITCH over the buckets, one PCG pass per branch
+    cudaGraphNodeParams sp = {};
+    if (e == cudaSuccess) {
+      sp.type = cudaGraphNodeTypeConditional;
+      sp.conditional.handle = hs;
+      sp.conditional.type = cudaGraphCondTypeSwitch;
+      sp.conditional.size = (unsigned)nb;
+      e = cudaGraphAddNode(&snode, body, &bnode, 1, &sp);
+    }
+    for (int k = 0; k < nb && e == cudaSuccess; ++k)
+      e = capture(sp.conditional.phGraph_out[k], nullptr, 0,
+                  [&] { pass(std::min(cap, 2 * (kMinBucketItems << k)), loop); });
+    // 3. loop control after the pass
+    if (e == cudaSuccess) e = capture(body, &snode, 1, [&] { loop_ctl(hw, dn, st, c->maxiter, shared_budget, s); });
   }
-  // 1. the bucket of this pass
-  if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    loop_bucket(hs, dn, st, kMinBucketItems, nb, s);
-    cudaGraph_t g1 = nullptr;
-    e = cudaStreamEndCapture(s, &g1);
-  }
-  size_t nn = 1;
-  if (e == cudaSuccess) e = cudaGraphGetNodes(body, &bnode, &nn);
-  // 2. SWITCH over the buckets, one PCG pass per branch
-  cudaGraphNodeParams sp = {};
-  if (e == cudaSuccess) {
-    sp.type = cudaGraphNodeTypeConditional;
-    sp.conditional.handle = hs;
-    sp.conditional.type = cudaGraphCondTypeSwitch;
-    sp.conditional.size = (unsigned)nb;
-    e = cudaGraphAddNode(&snode, body, &bnode, 1, &sp);
-  }
-  for (int k = 0; k < nb && e == cudaSuccess; ++k) {
-    e = cudaStreamBeginCaptureToGraph(s, sp.conditional.phGraph_out[k], nullptr, nullptr, 0,
-                                      cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) break;
-    pass(std::min(cap, 2 * (kMinBucketItems << k)));
-    cudaGraph_t gk = nullptr;
-    e = cudaStreamEndCapture(s, &gk);
-  }
-  // 3. loop control after the pass
-  if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, &snode, nullptr, 1, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    loop_ctl(hw, dn, st, c->maxiter, shared_budget, s);
-    cudaGraph_t g3 = nullptr;
-    e = cudaStreamEndCapture(s, &g3);
-  }
+  lg.launches = (c->kinetic_only ? 5 : 7) + (nb > 1 ? 2 : 0);
   c->stats = saved;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&lg.exec, lg.graph, 0);
   if (e != cudaSuccess) {
@@ -653,7 +685,7 @@ void loop_stats(wb_ctx* c, int passes, int launches_per_pass) {
 // at most n_dfpt_maxiter passes like the reference's PCG) and x += d in FP64;
 // at most kMaxRefinements residuals.  X holds the initial guess on entry
 // (dfpt_module.f90:348) and the solution on exit.
-int cg_mixed(wb_ctx* c, int mb, double tr2, int nsplit, int* iters_out) {
+int cg_mixed(wb_ctx* c, int mb, double tr2, int* iters_out) {
   cudaStream_t s = c->stream;
   const int npw = c->npw, nocc = c->nocc, nsys = mb * nocc;
   const long ld = npw;
@@ -671,15 +703,16 @@ int cg_mixed(wb_ctx* c, int mb, double tr2, int nsplit, int* iters_out) {
                                     c->items_in.p, c->nact_in.p, c->conv_in.p, c->rho_in.p, c->rho0.p,
                                     c->part32.p, c->C32.p,    c->ecol32.p, st,          (const void*)(intptr_t)cap};
     const int* dn = c->nact_in.as<int>();
-    rc = capture_loop(c, c->loop32, key, tr2, cap, dn, st, true, [&](int nmax) {
+    rc = capture_loop(c, c->loop32, key, tr2, cap, dn, st, true, [&](int nmax, CgLoop loop) {
       apply_A32(c, c->P32.as<float2>(), c->T32.as<float2>(), c->act_in.as<int>(), c->items_in.as<int2>(), nmax,
                 nsplit32, dn);
+      loop.act = c->act_in.as<int>();
+      loop.items = c->items_in.as<int2>();
+      loop.nact = c->nact_in.as<int>();
       cg_step32(c->act_in.as<int>(), nmax, c->d32.as<float2>(), c->g32.as<float2>(), c->P32.as<float2>(),
                 c->T32.as<float2>(), c->iprec.as<double>(), nocc, c->rho_in.as<double>(),
                 c->conv_in.as<unsigned char>(), 0, c->maxiter, kInnerRhoReduction, c->rho0.as<double>(), tr2, npw,
-                ld, s, dn, st + 1);
-      cg_compact(c->conv_in.as<unsigned char>(), cap, c->act_in.as<int>(), c->items_in.as<int2>(),
-                 c->nact_in.as<int>(), nullptr, s, st);
+                ld, s, dn, st + 1, &loop);
     });
     if (rc) return rc;
     loop_init(st, nsys, true, s);
@@ -696,7 +729,7 @@ int cg_mixed(wb_ctx* c, int mb, double tr2, int nsplit, int* iters_out) {
   cg_compact(conv, nsys, act, items, c->nact.as<int>(), c->nact_host, s);
   int nact = nsys, inner_total = 0;
   for (int outer = 0; outer < kMaxRefinements; ++outer) {
-    apply_A(c, X, T, act, items, nact, nsys, nsplit);                    // FP64 A x
+    apply_A(c, X, T, act, items, nact);                                  // FP64 A x
     {
       Stage g(c, WB_STAGE_CG, 2, nact);
       refine_residual(act, nact, B, T, c->iprec.as<double>(), nocc, tr2, conv, c->rho0.as<double>(),
@@ -753,7 +786,7 @@ int cg_mixed(wb_ctx* c, int mb, double tr2, int nsplit, int* iters_out) {
     Stage g(c, WB_STAGE_CG, 1, mb);
     count_unconverged(conv, nocc, mb, c->unconv.as<int>(), s);
   }
-  if (graph) loop_stats(c, inner_total, c->kinetic_only ? 6 : 9);
+  if (graph) loop_stats(c, inner_total, c->loop32.slot[c->loop32.last].launches);
   *iters_out = inner_total;
   if (c->umma) {  // a bounded wait of a tensor-core GEMM that ran out leaves its code here
     const int e = c->nact_host[1];
@@ -813,7 +846,7 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
   const double* Wevc = c->W.as<double>() + (size_t)c->nkb * K;
   int rc0 = autotune64(c, nsys);
   if (rc0) return rc0;
-  const int nsplit = gemm_tn_splits(c->nproj, nsys, K, c->tune.dmma_ctas);
+  const int nsplit = gemm_tn_plan(nocc, nsys, K, c->tune.dmma_ctas);
   {
     Stage g(c, WB_STAGE_OTHER, 4, nsys);
     gemm_tn(Wevc, K, nocc, (const double*)B, 2 * ld, nullptr, nsys, K, nsplit, c->part.as<double>(), s);
@@ -831,7 +864,7 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
   // 6. PCG                                           (dfpt_module.f90:350-361)
   int iters = 0;
   if (tr2 >= 0.0 && c->precision == WB_PRECISION_MIXED) {
-    int rc = cg_mixed(c, mb, tr2, nsplit, &iters);
+    int rc = cg_mixed(c, mb, tr2, &iters);
     if (rc) return rc;
   } else if (tr2 >= 0.0) {
     unsigned char* conv = c->conv.as<unsigned char>();
@@ -842,7 +875,7 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
       cg_reset(conv, nsys, s);
       cg_compact(conv, nsys, act, items, c->nact.as<int>(), c->nact_host, s);
     }
-    apply_A(c, X, T, act, items, nsys, nsys, nsplit);            // :127
+    apply_A(c, X, T, act, items, nsys);                          // :127
     {
       Stage g(c, WB_STAGE_CG, 1, nsys);
       sub_into(T, B, G, npw, nsys, ld, s);                       // :130-138
@@ -856,16 +889,17 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
     }
     if (graph) {                                                 // :146-330 as one graph launch
       const int cap = c->cap_nsys;
-      const int nsplit_cap = gemm_tn_splits(c->nproj, cap, K, c->tune.dmma_ctas);
       int* st = c->loopst.as<int>();
       const int* dn = c->nact.as<int>();
       std::vector<const void*> key = {B, X, G, T, c->sticks.p, act, items, dn, conv, c->rho.p, c->part.p, c->C.p,
                                       c->ecol.p, st, (const void*)(intptr_t)cap};
-      int rc = capture_loop(c, c->loop64, key, tr2, cap, dn, st, false, [&](int nmax) {
-        apply_A(c, B, T, act, items, nmax, cap, nsplit_cap, dn);
+      int rc = capture_loop(c, c->loop64, key, tr2, cap, dn, st, false, [&](int nmax, CgLoop loop) {
+        apply_A(c, B, T, act, items, nmax, dn);
+        loop.act = act;
+        loop.items = items;
+        loop.nact = c->nact.as<int>();
         cg_step(act, nmax, X, G, B, T, c->iprec.as<double>(), nocc, c->rho.as<double>(), conv, 0, c->maxiter, tr2,
-                npw, ld, s, dn, st + 1);
-        cg_compact(conv, cap, act, items, c->nact.as<int>(), nullptr, s, st);
+                npw, ld, s, dn, st + 1, &loop);
       });
       if (rc) return rc;
       loop_init(st, nsys, true, s);
@@ -873,7 +907,7 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
       WB_CU(cudaMemcpyAsync(c->loop_host, st, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
       // read after the batch's final wait (pending_loop_stats): no host round
       // trip between the PCG graph and the density stage
-      c->loop_pending = c->kinetic_only ? 6 : 9;
+      c->loop_pending = c->loop64.slot[c->loop64.last].launches;
     }
     for (int it = 1; !graph && it <= c->maxiter; ++it) {        // :146
       WB_CU(cudaStreamSynchronize(s));
@@ -881,7 +915,7 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
       iters = it;
       if (nact == 0) break;                                      // :222
       c->stats.cg_active_sum += nact;
-      apply_A(c, B, T, act, items, nact, nsys, nsplit);          // :251
+      apply_A(c, B, T, act, items, nact);                        // :251
       {
         Stage g(c, WB_STAGE_CG, 2, nact);
         // :253-329, then iteration it + 1's :146-222
@@ -1044,8 +1078,11 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
       cudaMallocHost(&c->nact_host, sizeof(int) * 4) != cudaSuccess ||
-      cudaMallocHost(&c->loop_host, sizeof(int) * 8) != cudaSuccess || c->loopst.ensure(sizeof(int) * 8) != 0 ||
+      cudaMallocHost(&c->loop_host, sizeof(int) * 8) != cudaSuccess || c->loopst.ensure(sizeof(int) * kLoopInts) != 0 ||
       cudaEventCreate(&c->tev0) != cudaSuccess || cudaEventCreate(&c->tev1) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->side_ev[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->side_ev[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->wait_ev, cudaEventBlockingSync | cudaEventDisableTiming) != cudaSuccess)
     return bail(fail(WB_ERR_CUDA, "stream/event creation failed"));
   c->npw = s->npw;
@@ -1070,10 +1107,6 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
   c->omega = s->omega;
   c->wk = s->wk;
   c->alpha = s->alpha_pv;
-  // FP64 bra-ket operand prefetch: two k steps ahead for few projectors (64 at
-  // the c2 cell: 4.3 -> 3.3 ms per m = 16 call), one for many (208 at the 108^3
-  // cell, where the extra registers cost more: 222 -> 242 ms)
-  c->tune.dmma_pf = c->nproj <= 96 ? 2 : 1;
   // fractional occupations (Tools/set_nbndocc.f90:58-69): nbnd_occ_full is the
   // highest band occupied above 1 - docc_thr; the correction of dfpt_module.f90:
   // 363-398 needs non-degenerate energies wherever the occupations differ (:387)
@@ -1156,6 +1189,7 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
     if (c->nkb) std::memcpy(dd.data(), s->deeq, sizeof(double) * c->nkb * c->nkb);
     if ((rc = upload(dd.data(), dd.size(), c->D))) return bail(rc);
   }
+  la_setup();
   if (c->rt) rt_setup(c->geo);
   else fft_setup(N);
   c->fa.n = N;
@@ -1214,6 +1248,9 @@ int wb_ctx_destroy(wb_ctx* c) {
   if (c->tev1) cudaEventDestroy(c->tev1);
   if (c->wait_ev) cudaEventDestroy(c->wait_ev);
   if (c->pin) cudaFreeHost(c->pin);
+  for (cudaEvent_t e : c->side_ev)
+    if (e) cudaEventDestroy(e);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -1281,7 +1318,7 @@ int wb_get_tuning(const wb_ctx* c, wb_tuning* out) {
   out->tuned_fp64 = c->tune.done64;
   out->tuned_mixed = c->tune.done32;
   out->dmma_ctas_per_sm = c->tune.dmma_ctas;
-  out->dmma_prefetch = c->tune.dmma_pf;
+  out->dmma_prefetch = kDmmaAhead;
   out->tc_braket_ctas_per_sm = c->tune.umma_ctas;
   out->tc_update_systems = c->tune.update_nj;
   out->plane_fused_fp64 = out->plane_fused_mixed = c->rt ? 0 : 1;
@@ -1361,21 +1398,25 @@ struct Carve {
   }
 };
 
+constexpr int kNoallocCtas = 2;  // the built-in split target
+
 struct NoallocWs {
   double2 *aux, *dvbox, *B, *X, *G, *T, *sticks, *sticks2, *acc;
   double *part, *C, *rho, *ecol, *epcol;
   unsigned char* conv;
   int *act, *nact, *unconv;
   int2 *items, *items_pp, *items_pk;
+  bool plan;   // the bra-kets split as the other entry points' do; else nsplit ways
   int nsplit;
 };
 
-void noalloc_layout(const wb_ctx* c, int mb, Carve& cv, NoallocWs& w) {
+void noalloc_layout(const wb_ctx* c, int mb, bool plan, Carve& cv, NoallocWs& w) {
   const size_t nsys = (size_t)mb * c->nocc;
   const size_t npw = c->npw;
   const size_t stk1 = (size_t)c->nz * c->st.nst;
   const size_t mp = ((size_t)mb + 1) / 2;
   const size_t nitems = std::max<size_t>({(nsys + 1) / 2, (size_t)mb * c->npv, mp});
+  w.plan = plan;
   w.nsplit = gemm_tn_splits(c->nproj, (int)nsys, 2 * c->npw);
   w.aux = cv.take<double2>(npw * mb);
   w.dvbox = cv.take<double2>((size_t)c->nnr * mp);
@@ -1386,7 +1427,9 @@ void noalloc_layout(const wb_ctx* c, int mb, Carve& cv, NoallocWs& w) {
   w.sticks = cv.take<double2>(stk1 * nitems);
   w.sticks2 = cv.take<double2>(stk1 * mp);
   w.acc = cv.take<double2>((size_t)c->nnr * mp);
-  w.part = cv.take<double>((size_t)w.nsplit * nsys * c->nproj);
+  w.part = cv.take<double>(plan ? std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw, kNoallocCtas),
+                                           gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw, kNoallocCtas))
+                                : (size_t)w.nsplit * nsys * c->nproj);
   w.C = cv.take<double>(nsys * c->nproj);
   w.rho = cv.take<double>(nsys);
   w.ecol = cv.take<double>(nsys);
@@ -1429,8 +1472,9 @@ void noalloc_apply_A(wb_ctx* c, const NoallocWs& w, const double2* Xv, double2* 
     fft_plane_vloc(c->fa, w.sticks, nit, c->vs.as<double>());
     fft_zfwd_hpsi(c->fa, w.sticks, items, nit, Xv, Tv, ld, c->g2kin.as<double>(), w.ecol);
   }
-  gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, w.nsplit, w.part, s);
-  gamma_reduce(w.part, w.nsplit, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(), nkb, c->alpha,
+  const int ns = w.plan ? gemm_tn_plan(M, n, K, kNoallocCtas) : w.nsplit;
+  gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, ns, w.part, s);
+  gamma_reduce(w.part, ns, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(), nkb, c->alpha,
                w.C, s);
   gemm_nn(Wsub, K, M, w.C, (double*)Tv, 2 * ld, cols, n, K, 1.0, s);
 }
@@ -1453,8 +1497,9 @@ int noalloc_run(wb_ctx* c, const NoallocWs& w, int mb, const double2* dvg, long 
   fft_plane_rhs(c->fa, c->evcr.as<double2>(), w.dvbox, npv, mb, w.sticks);
   fft_zfwd_store(c->fa, w.sticks, w.items_pk, mb * npv, w.B, ld);
   const double* Wevc = c->W.as<double>() + (size_t)c->nkb * K;
-  gemm_tn(Wevc, K, nocc, (const double*)w.B, 2 * ld, nullptr, nsys, K, w.nsplit, w.part, s);
-  gamma_reduce(w.part, w.nsplit, nocc, nsys, Wevc, K, (const double*)w.B, 2 * ld, nullptr, nullptr, 0, 1.0, w.C, s);
+  const int ns = w.plan ? gemm_tn_plan(nocc, nsys, K, kNoallocCtas) : w.nsplit;
+  gemm_tn(Wevc, K, nocc, (const double*)w.B, 2 * ld, nullptr, nsys, K, ns, w.part, s);
+  gamma_reduce(w.part, ns, nocc, nsys, Wevc, K, (const double*)w.B, 2 * ld, nullptr, nullptr, 0, 1.0, w.C, s);
   gemm_nn(Wevc, K, nocc, w.C, (double*)w.B, 2 * ld, nullptr, nsys, K, -1.0, s);
   precondition(w.B, w.X, c->iprec.as<double>(), nocc, npw, nsys, ld, s);
   int iters = 0;
@@ -1515,9 +1560,18 @@ extern "C" int wb_apply_operator_device_noalloc(wb_ctx* c, int m, const double* 
     return fail(WB_ERR_ARG, "m = " + std::to_string(m) + " perturbations do not fit the allocation-free entry "
                 "point's scratch of " + std::to_string((size_t)WB_NOALLOC_SCRATCH_BYTES) +
                 " bytes (WB_NOALLOC_SCRATCH_BYTES): use fewer perturbations per call");
+  // the split plan of the other entry points where its partial sums fit too, so
+  // that up to 64 systems give their bits; a call that fits only without them runs
+  // with fewer splits
   Carve probe{nullptr};
   NoallocWs w{};
-  noalloc_layout(c, std::max(m, 1), probe, w);
+  bool plan = true;
+  noalloc_layout(c, std::max(m, 1), plan, probe, w);
+  if (probe.off > (size_t)WB_NOALLOC_SCRATCH_BYTES) {
+    plan = false;
+    probe = Carve{nullptr};
+    noalloc_layout(c, std::max(m, 1), plan, probe, w);
+  }
   if (probe.off > (size_t)WB_NOALLOC_SCRATCH_BYTES)
     return fail(WB_ERR_ARG, "this call needs " + std::to_string(probe.off) + " bytes of scratch; the allocation-free "
                 "entry point has " + std::to_string((size_t)WB_NOALLOC_SCRATCH_BYTES) +
@@ -1530,7 +1584,7 @@ extern "C" int wb_apply_operator_device_noalloc(wb_ctx* c, int m, const double* 
   c->stats.m = m;
   if (m == 0) return WB_OK;
   Carve cv{base};
-  noalloc_layout(c, m, cv, w);
+  noalloc_layout(c, m, plan, cv, w);
   if (ld_dng > c->npw)
     WB_CU(cudaMemset2DAsync(reinterpret_cast<double2*>(dng) + c->npw, sizeof(double2) * ld_dng, 0,
                             sizeof(double2) * (ld_dng - c->npw), m, c->stream));

@@ -88,6 +88,7 @@ struct wb_ctx {
     cudaGraphExec_t exec = nullptr;
     std::vector<const void*> key;
     double tr2 = 0.0;
+    int launches = 0;  // per pass
     void release() {
       if (exec) cudaGraphExecDestroy(exec);
       if (graph) cudaGraphDestroy(graph);
@@ -114,10 +115,12 @@ struct wb_ctx {
   // autotuned launch shapes (set on the first batch of each form, then fixed)
   struct Tune {
     int on = 1, done64 = 0, done32 = 0;
-    int dmma_ctas = 2, dmma_pf = 1, umma_ctas = 2, update_nj = 0;
+    int dmma_ctas = 2, umma_ctas = 2, update_nj = 0;
     float ms = 0.f;
   } tune;
   cudaEvent_t tev0 = nullptr, tev1 = nullptr;
+  cudaStream_t side = nullptr;  // second branch of a captured PCG pass
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
   cudaEvent_t wait_ev = nullptr;  // blocking-sync event of the calls' waits (wb_wait)
   // pinned staging of a batch's small host transfers (unconverged counts, item
   // tables): copies from or to pageable memory would wait for the stream by
@@ -136,7 +139,7 @@ struct wb_ctx {
     pin_bytes = b;
     return 0;
   }
-  DBuf loopst;               // int[8] loop state (wb_la.cu loop_init / loop_ctl)
+  DBuf loopst;               // int[kLoopInts] loop state (wb_la.cu loop_init / loop_ctl)
   int* loop_host = nullptr;  // pinned copy of it
   int loop_pending = 0;      // launches per pass of a graph run whose counters await the batch's wait
   // tensor-core GEMMs of the mixed form: W split into bf16 hi/lo tiles, and the

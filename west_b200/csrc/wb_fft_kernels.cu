@@ -281,6 +281,7 @@ struct EpiDng {
 // ---------------------------------------------------------------------------
 // x-y plane passes (phases and layout: wb_plane.cuh)
 // ---------------------------------------------------------------------------
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory of one CTA
 template <int N, class C>
 constexpr size_t psmem() { return sizeof(C) * CPlane<N, true>::SIZE; }
 
@@ -298,7 +299,7 @@ constexpr int plane_threads() {
   if (N <= 64) return 256;
   if (N <= 72) return 352;
   if (N <= 80) return 416;
-  if (N <= 96) return 576;
+  if (N <= 96) return sizeof(C) == 16 ? 576 : 512;
   return 512;
 }
 template <int N, class C>
@@ -347,19 +348,53 @@ WB_DEV void plane_forward(C* pl, const TW& tw, C* sz, const StickTab& st, const 
 // zeroed, scattered and gathered the plane and read their twiddles from shared
 // memory per lane: 64^3 1.30 us (was 1.65) in FP64, 0.71 (0.92) in FP32; 80^3
 // 3.1 (5.2) in FP64; 108^3 9.8 (14.0) and 4.8 (7.0); 48^3 1.1 (1.8).
-template <int N, bool PR, class C>
+//
+// STAGED: a persistent CTA that runs over the units (plane, item) with the next
+// unit's sticks copied into a shared-memory stage while it works on one, where
+// one CTA fills an SM and the stage fits beside its plane.  Without it each CTA
+// begins with two dependent trips to L2 or DRAM (3,500 of an FP64 108^3 plane's
+// 24,400 cycles) and ends in a launch gap that nothing hides: 9.77 -> 9.14 us per
+// item.  With several CTAs per SM the others hide both and the stage only costs
+// (FP32 64^3 0.71 -> 0.76 us, 108^3 4.77 -> 4.92).
+template <int N, bool PR, class C, bool STAGED>
 __global__ void __launch_bounds__(plane_threads<N, C>(), plane_blocks<N, C>()) k_plane_vloc(
     C* __restrict__ sticks, StickTab st, const real_t<C>* __restrict__ vs, const __grid_constant__ TwParam<N, C> tw,
-    const int* dn) {
-  if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;
+    int nitems, const int* dn) {
   constexpr int NT = plane_threads<N, C>();
   C* pl = smem_tw<C>();
   const CPlane<N, PR> g(st.ncols, st.xhi + 1);
-  const int z = blockIdx.x, item = blockIdx.y;
-  C* sz = sticks + ((long)item * N + z) * st.nst;
-  plane_inverse(pl, tw, sz, st, g, NT);
-  plane_row_vloc<FftSplit<N>::N2>(pl, tw, vs + (long)z * N * N, g, NT);
-  plane_forward(pl, tw, sz, st, g, NT);
+  if constexpr (STAGED) {
+    const int units = dev_count<true>(dn, nitems) * N;  // unit = item * N + z
+    C* stage = pl + CPlane<N, PR>::SIZE;
+    auto fetch = [&](int u) {
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(sticks + (long)u * st.nst);
+      unsigned char* dst = reinterpret_cast<unsigned char*>(stage);
+      for (int b = threadIdx.x * 16; b < st.nst * (int)sizeof(C); b += NT * 16)
+        cp_async_elem(reinterpret_cast<double2*>(dst + b), reinterpret_cast<const double2*>(src + b));
+    };
+    int u = blockIdx.x;
+    if (u < units) fetch(u);
+    for (; u < units; u += gridDim.x) {
+      cp_async_wait_all();
+      __syncthreads();  // the stage is full; the last unit's column pass is done with the plane
+      plane_col_in<FftSplit<N>::N1>(pl, tw, stage, st.cmap, g, NT);
+      __syncthreads();
+      if (u + (int)gridDim.x < units) fetch(u + gridDim.x);
+      plane_col_mid_inv<FftSplit<N>::N2>(pl, g, NT);
+      __syncthreads();
+      plane_row_in<FftSplit<N>::N1>(pl, tw, g, NT);
+      __syncthreads();
+      plane_row_vloc<FftSplit<N>::N2>(pl, tw, vs + (long)(u % N) * N * N, g, NT);
+      plane_forward(pl, tw, sticks + (long)u * st.nst, st, g, NT);
+    }
+  } else {
+    if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;
+    const int z = blockIdx.x, item = blockIdx.y;
+    C* sz = sticks + ((long)item * N + z) * st.nst;
+    plane_inverse(pl, tw, sz, st, g, NT);
+    plane_row_vloc<FftSplit<N>::N2>(pl, tw, vs + (long)z * N * N, g, NT);
+    plane_forward(pl, tw, sz, st, g, NT);
+  }
 }
 
 // sticks -> full real-space box (complex: two real functions), no scaling
@@ -534,13 +569,15 @@ struct FftN {
     smem(k_zfwd<N, PR, double2, EpiStore>, zsmem<N>());
     smem(k_zfwd<N, PR, double2, EpiHpsi>, zsmem<N>());
     smem(k_zfwd<N, PR, double2, EpiDng>, zsmem<N>());
-    smem(k_plane_vloc<N, PR, double2>, psmem<N, double2>());
+    smem(k_plane_vloc<N, PR, double2, false>, psmem<N, double2>());
+    if constexpr (plane_blocks<N, double2>() == 1) smem(k_plane_vloc<N, PR, double2, true>, kMaxSmem);
+    if constexpr (plane_blocks<N, float2>() == 1) smem(k_plane_vloc<N, PR, float2, true>, kMaxSmem);
     smem(k_plane_inv_box<N, PR>, psmem<N, double2>());
     smem(k_plane_rhs<N, PR>, psmem<N, double2>());
     smem(k_plane_drho<N, PR>, psmem<N, double2>());
     smem(k_zinv<N, PR, float2>, zsmem<N, float2>());
     smem(k_zfwd<N, PR, float2, EpiHpsi32>, zsmem<N, float2>());
-    smem(k_plane_vloc<N, PR, float2>, psmem<N, float2>());
+    smem(k_plane_vloc<N, PR, float2, false>, psmem<N, float2>());
   }
   static void setup() {
     setup_pr<false>();
@@ -565,9 +602,17 @@ struct FftN {
     if (nitems <= 0) return;
     constexpr size_t ps = psmem<N, C>();
     constexpr int nt = plane_threads<N, C>();
-    const dim3 g(N, nitems);
-    if (f.st.prune) k_plane_vloc<N, true, C><<<g, nt, ps, f.stream>>>(sticks, f.st, vs, tw_param<C>(), f.dcount);
-    else k_plane_vloc<N, false, C><<<g, nt, ps, f.stream>>>(sticks, f.st, vs, tw_param<C>(), f.dcount);
+    if constexpr (plane_blocks<N, C>() == 1) {
+      const size_t staged = ps + sizeof(C) * f.st.nst;
+      if (staged <= kMaxSmem) {
+        const int grid = std::min(nitems * N, sm_count());
+        auto k = f.st.prune ? k_plane_vloc<N, true, C, true> : k_plane_vloc<N, false, C, true>;
+        k<<<grid, nt, staged, f.stream>>>(sticks, f.st, vs, tw_param<C>(), nitems, f.dcount);
+        return;
+      }
+    }
+    auto k = f.st.prune ? k_plane_vloc<N, true, C, false> : k_plane_vloc<N, false, C, false>;
+    k<<<dim3(N, nitems), nt, ps, f.stream>>>(sticks, f.st, vs, tw_param<C>(), nitems, f.dcount);
   }
   template <class C, class F, class Epi>
   static void zfwd_t(const F& f, const C* sticks, const int2* items, int nitems, Epi epi) {

@@ -89,6 +89,9 @@ void rt_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evcr
                    int mb, double2* acc, double scale, double2* osticks);
 void rt_setup(const RtGeo& g);
 
+// SMs of the current device
+int sm_count();
+
 bool fft_supported(int n);
 // the split n = a * b of a compiled edge's line transforms: the plane kernels
 // keep y = k1 + a k2 of real space at row b k1 + k2 (0, 0 for other edges)
@@ -134,22 +137,46 @@ void fft_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evc
 // Split-K plans of the bra-ket GEMMs, host and device: a graph replay sizes its
 // split grid for the largest plan and every CTA derives the plan of the device
 // column count itself, so both paths split the same count the same way.
-constexpr int kDmmaTile = 32;  // DMMA bra-ket CTA tile (rows and columns)
-// split count of the DMMA bra-ket: about 2 * 148 * ctas_per_sm CTAs (4 warps each)
+// gemm_tn_splits: splits of a caller with a fixed part buffer (about 2 * 148 *
+// ctas_per_sm CTAs of 32 x 32 tiles, at least 512 k each).
 __host__ __device__ inline int gemm_tn_splits(int M, int ncol, int K, int ctas_per_sm = 2) {
-  const int tiles = ((M + kDmmaTile - 1) / kDmmaTile) * ((ncol + kDmmaTile - 1) / kDmmaTile);
+  const int tiles = ((M + 31) / 32) * ((ncol + 31) / 32);
   int ns = (2 * 148 * ctas_per_sm + tiles - 1) / (tiles > 0 ? tiles : 1);
   const int maxs = (K + 511) / 512;
   if (ns > maxs) ns = maxs;
   if (ns < 1) ns = 1;
   return ns;
 }
+// k's of one split: a multiple of the pair width and of 16
+__host__ __device__ inline int gemm_tn_chunk(int K, int nsplit) { return ((K + nsplit - 1) / nsplit + 15) / 16 * 16; }
+// gemm_tn_plan: splits of the PCG's bra-kets.  Up to kDmmaSmall columns the 32 x
+// 32 tile runs and a CTA's serial chain is the time: about two CTAs per SM, at
+// least 128 k each.  Above, tiles of 64 columns and 64 rows (112 where there are
+// more): about ctas_per_sm CTAs per SM over the whole grid, at least 256 k each.
+constexpr int kDmmaAhead = 2;   // stages of operands a CTA loads ahead of its MMAs, at least
+constexpr int kDmmaSmall = 64;
+__host__ __device__ inline int gemm_tn_plan(int M, int ncol, int K, int ctas_per_sm) {
+  const bool small = ncol <= kDmmaSmall;
+  const int tr = small ? 32 : M > 64 ? 112 : 64, tj = small ? 32 : 64;
+  const int tiles = ((M + tr - 1) / tr) * ((ncol + tj - 1) / tj);
+  const int target = small ? 2 * 148 : 148 * ctas_per_sm;
+  int ns = target / (tiles > 0 ? tiles : 1);  // not over the target: a few CTAs more would be a whole wave
+  const int maxs = K / (small ? 128 : 256);
+  if (ns > maxs) ns = maxs;
+  if (ns < 1) ns = 1;
+  return ns;
+}
+// the largest plan of any count up to ncol that runs the same tile
+__host__ __device__ inline int gemm_tn_plan_max(int M, int ncol, int K, int ctas_per_sm) {
+  return gemm_tn_plan(M, ncol <= kDmmaSmall ? 1 : kDmmaSmall + 1, K, ctas_per_sm);
+}
 // part doubles for any column count up to nsys and any target up to ctas_max
 size_t gemm_tn_part_doubles(int M, int nsys, int K, int ctas_max);
-// with dn, ctas selects the device plan (nsplit is then ignored); prefetch: k
-// steps between an operand load and its MMAs (1 or 2)
+// with dn, ctas selects the device plan (nsplit is then ignored)
 void gemm_tn(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol, int K,
-             int nsplit, double* part, cudaStream_t s, const int* dn = nullptr, int ctas = 2, int prefetch = 1);
+             int nsplit, double* part, cudaStream_t s, const int* dn = nullptr, int ctas = 2);
+// opts the GEMM kernels into their shared memory on the current device
+void la_setup();
 // S = 2 sum_s part - W0 X0 (Gamma bra-ket, glbrak.f90:39-40), then
 // C[j][r] = sum_{r'<nkb} D[r][r'] S[j][r'] for r < nkb, alpha S[j][r] otherwise
 void gamma_reduce(const double* part, int nsplit, int M, int ncol, const double* W, long ldw, const double* X,
@@ -183,18 +210,30 @@ void cg_prec_rho(const int* act, int nact, const double2* g, double2* P, const d
 // nact_host may be null (no host copy); nsys_dev, if given, overrides nsys
 void cg_compact(const unsigned char* conv, int nsys, int* act, int2* items, int* nact_dev, int* nact_host,
                 cudaStream_t s, const int* nsys_dev = nullptr);
+// Loop state a captured PCG pass hands to its step kernel (wb_la.cu, CgTail):
+// the active list it rebuilds and, with ctl, the WHILE condition it sets.
+struct CgLoop {
+  int* act;
+  int2* items;
+  int* nact;
+  int* st;  // int[kLoopInts]
+  cudaGraphConditionalHandle cond;
+  int ctl, inner;
+};
+constexpr int kLoopInts = 12;
 // One PCG step after the operator: the update of iteration `iter` and, unless
 // iter == maxiter, the preconditioning / rho / convergence test / direction of
-// iteration iter + 1 (the iteration comes from *iter_dev when given).
+// iteration iter + 1 (the iteration comes from *iter_dev when given); with loop,
+// also the end of the pass.
 void cg_step(const int* act, int nact, double2* x, double2* g, double2* P, const double2* T, const double* iprec,
              int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double tr2, int npw, long ld,
-             cudaStream_t s, const int* dn = nullptr, const int* iter_dev = nullptr);
+             cudaStream_t s, const int* dn = nullptr, const int* iter_dev = nullptr, const CgLoop* loop = nullptr);
 void cg_step32(const int* act, int nact, float2* x, float2* g, float2* P, const float2* T, const double* iprec,
                int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double eta, const double* rel,
                double floor, int npw, long ld, cudaStream_t s, const int* dn = nullptr,
-               const int* iter_dev = nullptr);
+               const int* iter_dev = nullptr, const CgLoop* loop = nullptr);
 void count_unconverged(const unsigned char* conv, int nocc, int mb, int* out, cudaStream_t s);
-// loop state of the graph-captured PCG loops: int st[8] (wb_la.cu)
+// loop state of the graph-captured PCG loops: int st[kLoopInts] (wb_la.cu)
 void loop_init(int* st, int nsys, bool reset_totals, cudaStream_t s);
 void loop_ctl(cudaGraphConditionalHandle h, const int* nact, int* st, int maxiter, bool inner, cudaStream_t s);
 void loop_bucket(cudaGraphConditionalHandle h, const int* nact, int* st, int min_items, int nbuckets, cudaStream_t s);

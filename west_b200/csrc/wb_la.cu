@@ -12,270 +12,423 @@
 
 namespace wb {
 
+int sm_count() {
+  static int nsm = 0;
+  if (!nsm) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) !=
+                                                  cudaSuccess || nsm <= 0)
+      nsm = 148;
+  }
+  return nsm;
+}
+
+
 WB_DEV void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
 
+// cp.async of 16 or (rows that are not 16-byte aligned) twice 8 bytes; zeros
+// when !ok.  Copies are committed in groups, one per stage of a ring.
+WB_DEV void cp_pair(double* smem, const double* gmem, bool ok, bool al16) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  if (al16) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s + 8), "l"(gmem + 1), "r"(ok ? 8 : 0)
+                 : "memory");
+  }
+}
+WB_DEV void cp_one(double* smem, const double* gmem, bool ok) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0) : "memory");
+}
+WB_DEV void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT>
+WB_DEV void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
+
 // ---------------------------------------------------------------------------
 // part[s][j][r] = sum_{k in split s} W[r][k] X[col j][k]        (A^T B, split K)
-// CTA tile 32 r x 32 j, four warps interleave k in steps of 4 and are summed
-// through shared memory at the end.
+// A CTA of four warps takes TR rows r x TJ columns j; stages of KS k's of both
+// operands stream through a ring of ST buffers in shared memory by cp.async, so
+// a CTA has (ST - 1) stages in flight whatever its warps do.  Rows of KS + 4
+// doubles put the fragments of a half-warp (4 rows x 4 k) on distinct banks.
+//   64 x 64 (warps 2 x 2 of 32 x 32): the throughput form up to 64 rows; 16
+//     wavefronts per 64 cycles of DMMA and 0.125 bytes per flop from L2.  64 rows,
+//     1,200 columns, K = 16,880: 26 TFLOP/s of the pipe's 36.9 (16 before, with
+//     32 x 32 tiles whose warps read their operands from global memory).
+//   112 x 64 (each warp 112 x 16): more rows, split evenly over tiles (208 rows as
+//     2 x 104), so that X is read once per 112 rows: 208 rows, 160 columns, K =
+//     74,774: 21 TFLOP/s (14 before, 18 with 64 x 64 tiles).
+//   small tile (32 x 32, the four warps interleave k and are summed at the end,
+//     KS = 64): few columns, where the time is the latency of one CTA's chain.
+// K is even and a stage reads pairs of k; al16: rows are 16-byte aligned.
 // ---------------------------------------------------------------------------
-constexpr int TN_T = 32;
-constexpr int TN_W = 4;
+template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
+struct TnTile {
+  static constexpr int LD = KS + 4, ROWS = TR + TJ, STAGE = ROWS * LD;
+  static constexpr int RG = TR / WR / 8, JG = TJ / WJ / 8;
+  static constexpr int SMEM = (int)sizeof(double) * (STAGE * ST > WK * TR * TJ ? STAGE * ST : WK * TR * TJ);
+  static_assert(WR * WJ * WK == 4, "four warps");
+};
 
-// PF: k steps between an operand load and the MMAs that use it (1 or 2: two
-// pay at 64 projectors, cost at 208; same sums in the same order either way)
-template <int PF>
-__global__ void __launch_bounds__(32 * TN_W) k_gemm_tn(const double* __restrict__ W, long ldw, int M,
-                                                       const double* __restrict__ X, long ldx,
-                                                       const int* __restrict__ cols, int ncol_host, const int* dn,
-                                                       int K, int kchunk, int ctas, double* __restrict__ part) {
-  __shared__ double red[TN_W][TN_T * TN_T];
+template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
+__global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ W, long ldw, int M,
+                                                 const double* __restrict__ X, long ldx,
+                                                 const int* __restrict__ cols, int ncol_host, const int* dn, int K,
+                                                 int kchunk, int ctas, int trows, int al16,
+                                                 double* __restrict__ part) {
+  using G = TnTile<TR, TJ, WR, WJ, WK, KS, ST>;
+  constexpr int LD = G::LD, RG = G::RG, JG = G::JG;
+  extern __shared__ __align__(16) double tn_sm[];
   const int ncol = dev_count(dn, ncol_host);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lr = lane >> 2, lk = lane & 3;
-  const int r0 = blockIdx.x * TN_T, j0 = blockIdx.y * TN_T, split = blockIdx.z;
+  const int r0 = blockIdx.x * trows, j0 = blockIdx.y * TJ, split = blockIdx.z;
+  const int rend = min(M, r0 + trows);
   if (j0 >= ncol) return;
   if (dn) {  // the split plan of this column count
-    const int ns = gemm_tn_splits(M, ncol, K, ctas);
+    const int ns = gemm_tn_plan(M, ncol, K, ctas);
     if (split >= ns) return;
-    kchunk = ((K + ns - 1) / ns + 15) / 16 * 16;
+    kchunk = gemm_tn_chunk(K, ns);
   }
   const int kb = split * kchunk, ke = min(K, kb + kchunk);
-  const double* arow[4];
-  bool aok[4];
-  const double* bcol[4];
-  bool bok[4];
+  // copies: KS/2 pairs of k per row; a thread's pair index is fixed, its rows step
+  constexpr int PR = KS / 2, RSTEP = 128 / PR, NROW = G::ROWS / RSTEP;
+  static_assert(128 % PR == 0 && G::ROWS % RSTEP == 0, "copy shape");
+  const int kp = (tid % PR) * 2, row0 = tid / PR;
+  const double* src[NROW];
+  unsigned okm = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + i * 8 + lr;
-    aok[i] = r < M;
-    arow[i] = W + (long)(aok[i] ? r : 0) * ldw;
-    const int j = j0 + i * 8 + lr;
-    bok[i] = j < ncol;
-    const int c = bok[i] ? (cols ? cols[j] : j) : 0;
-    bcol[i] = X + (long)c * ldx;
-  }
-  double acc[4][4][2];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-  auto load = [&](int k, double* a, double* b) {
-    const int kk = k + lk;
-    const bool kok = kk < ke;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a[i] = (aok[i] && kok) ? __ldg(arow[i] + kk) : 0.0;
-      b[i] = (bok[i] && kok) ? __ldg(bcol[i] + kk) : 0.0;
-    }
-  };
-  auto mma_step = [&](const double* a, const double* b) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-  };
-  constexpr int KS = 4 * TN_W;  // k advanced per step (the CTA's warps interleave k)
-  const int k0 = kb + warp * 4;
-  if constexpr (PF == 1) {      // the next step's operands load while this step's MMAs run
-    double av[4], bv[4];
-    load(k0, av, bv);
-    for (int k = k0; k < ke; k += KS) {
-      double an[4], bn[4];
-      load(k + KS, an, bn);
-      mma_step(av, bv);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { av[i] = an[i]; bv[i] = bn[i]; }
-    }
-  } else {                      // two steps ahead; two steps per trip, the buffers swap roles
-    double a0[4], b0[4], a1[4], b1[4];
-    load(k0, a0, b0);
-    load(k0 + KS, a1, b1);
-    for (int k = k0; k < ke; k += 2 * KS) {
-      mma_step(a0, b0);         // step k, loaded two steps ago
-      load(k + 2 * KS, a0, b0);
-      if (k + KS >= ke) break;
-      mma_step(a1, b1);         // step k + KS
-      load(k + 3 * KS, a1, b1);
+  for (int i = 0; i < NROW; ++i) {
+    const int row = row0 + i * RSTEP;
+    src[i] = W;
+    if (row < TR) {
+      const int r = r0 + row;
+      if (r < rend) { src[i] = W + (long)r * ldw; okm |= 1u << i; }
+    } else {
+      const int j = j0 + row - TR;
+      if (j < ncol) { src[i] = X + (long)(cols ? cols[j] : j) * ldx; okm |= 1u << i; }
     }
   }
+  auto fetch = [&](int st, int k0) {
+    double* d = tn_sm + st * G::STAGE + row0 * LD + kp;
+    const int k = k0 + kp;
+    const bool kok = k < ke;
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int i = 0; i < NROW; ++i)
+      cp_pair(d + i * RSTEP * LD, src[i] + (kok ? k : 0), kok && (okm >> i & 1u), al16 != 0);
+  };
+  const int wk = warp % WK, wj = warp / WK % WJ, wr = warp / WK / WJ;
+  const int rb = wr * (TR / WR), jb = wj * (TJ / WJ);
+  // fragments of eight rows or columns beyond M or ncol are skipped, warp-uniformly
+  const int nr = min(RG, max(0, (rend - r0 - rb + 7) / 8)), nj = min(JG, max(0, (ncol - j0 - jb + 7) / 8));
+  double acc[RG][JG][2];
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+  for (int a = 0; a < RG; ++a)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) red[warp][(a * 8 + lr) * TN_T + b * 8 + 2 * lk + h] = acc[a][b][h];
-  __syncthreads();
-  for (int e = threadIdx.x; e < TN_T * TN_T; e += 32 * TN_W) {
-    double s = 0.0;
+    for (int b = 0; b < JG; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 #pragma unroll
-    for (int w = 0; w < TN_W; ++w) s += red[w][e];
-    const int r = r0 + e / TN_T, j = j0 + e % TN_T;
-    if (r < M && j < ncol) part[((long)split * ncol + j) * M + r] = s;
+  for (int st = 0; st < ST - 1; ++st) {
+    if (kb + st * KS < ke) fetch(st, kb + st * KS);
+    cp_commit();
+  }
+  int st = 0;
+  for (int k0 = kb; k0 < ke; k0 += KS) {
+    cp_wait<ST - 2>();
+    __syncthreads();
+    const int kn = k0 + (ST - 1) * KS;
+    if (kn < ke) fetch(st == 0 ? ST - 1 : st - 1, kn);
+    cp_commit();
+    const double* sw = tn_sm + st * G::STAGE + (rb + lr) * LD + wk * 4 + lk;
+    const double* sx = tn_sm + st * G::STAGE + (TR + jb + lr) * LD + wk * 4 + lk;
+    if (nr >= RG - 1 && nj == JG) {  // at most one fragment of zero rows
+#pragma unroll
+      for (int kk = 0; kk < KS; kk += 4 * WK) {
+        double av[RG], bv[JG];
+#pragma unroll
+        for (int i = 0; i < RG; ++i) av[i] = sw[i * 8 * LD + kk];
+#pragma unroll
+        for (int i = 0; i < JG; ++i) bv[i] = sx[i * 8 * LD + kk];
+#pragma unroll
+        for (int a = 0; a < RG; ++a)
+#pragma unroll
+          for (int b = 0; b < JG; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
+      }
+    } else if (nr > 0 && nj > 0) {
+#pragma unroll
+      for (int kk = 0; kk < KS; kk += 4 * WK) {
+        double bv[JG];
+#pragma unroll
+        for (int i = 0; i < JG; ++i) bv[i] = sx[i * 8 * LD + kk];
+#pragma unroll
+        for (int a = 0; a < RG; ++a)
+          if (a < nr) {
+            const double av = sw[a * 8 * LD + kk];
+#pragma unroll
+            for (int b = 0; b < JG; ++b)
+              if (b < nj) dmma(acc[a][b][0], acc[a][b][1], av, bv[b]);
+          }
+      }
+    }
+    st = st == ST - 1 ? 0 : st + 1;
+  }
+  cp_wait<0>();
+  if constexpr (WK == 1) {
+#pragma unroll
+    for (int b = 0; b < JG; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + jb + b * 8 + 2 * lk + h;
+        if (j >= ncol) continue;
+        double* o = part + ((long)split * ncol + j) * M + r0 + rb + lr;
+#pragma unroll
+        for (int a = 0; a < RG; ++a)
+          if (r0 + rb + a * 8 + lr < rend) o[a * 8] = acc[a][b][h];
+      }
+  } else {
+    static_assert(WK == 1 || (WR == 1 && WJ == 1), "k-interleaved warps share one tile");
+    __syncthreads();  // the ring becomes the warps' sums, [warp][j][r]
+    double* red = tn_sm + wk * TR * TJ;
+#pragma unroll
+    for (int a = 0; a < RG; ++a)
+#pragma unroll
+      for (int b = 0; b < JG; ++b)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) red[(b * 8 + 2 * lk + h) * TR + a * 8 + lr] = acc[a][b][h];
+    __syncthreads();
+    for (int e = tid; e < TR * TJ; e += 128) {
+      const int r = r0 + e % TR, j = j0 + e / TR;
+      if (r >= rend || j >= ncol) continue;
+      double sum = 0.0;
+#pragma unroll
+      for (int w = 0; w < WK; ++w) sum += tn_sm[w * TR * TJ + e];
+      part[((long)split * ncol + j) * M + r] = sum;
+    }
   }
 }
 
 size_t gemm_tn_part_doubles(int M, int nsys, int K, int ctas_max) {
   size_t best = 0;
-  for (int t = 1; t <= (nsys + TN_T - 1) / TN_T; ++t) {
-    const int n = std::min(nsys, t * TN_T);
-    for (int c = 1; c <= ctas_max; ++c) best = std::max(best, (size_t)gemm_tn_splits(M, n, K, c) * n * M);
+  for (int t = 1; t <= (nsys + 31) / 32; ++t) {
+    const int n = std::min(nsys, t * 32);
+    for (int c = 1; c <= ctas_max; ++c) best = std::max(best, (size_t)gemm_tn_plan(M, n, K, c) * n * M);
   }
   return best;
 }
 
+template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
+static void gemm_tn_launch(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol,
+                           int K, int nsplit, double* part, cudaStream_t s, const int* dn, int ctas, int al16) {
+  constexpr int SM = TnTile<TR, TJ, WR, WJ, WK, KS, ST>::SMEM;
+  auto k = k_gemm_tn<TR, TJ, WR, WJ, WK, KS, ST>;
+  const int tiles = (M + TR - 1) / TR, trows = ((M + tiles - 1) / tiles + 7) / 8 * 8;
+  dim3 grid(tiles, (ncol + TJ - 1) / TJ, nsplit);
+  k<<<grid, 128, SM, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, gemm_tn_chunk(K, nsplit), ctas, trows, al16, part);
+}
 void gemm_tn(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol, int K,
-             int nsplit, double* part, cudaStream_t s, const int* dn, int ctas, int prefetch) {
+             int nsplit, double* part, cudaStream_t s, const int* dn, int ctas) {
   if (ncol <= 0 || M <= 0) return;
-  if (dn) nsplit = gemm_tn_splits(M, 1, K, ctas);  // grid for the largest plan
-  int kchunk = (K + nsplit - 1) / nsplit;
-  kchunk = (kchunk + 15) / 16 * 16;
-  dim3 grid((M + TN_T - 1) / TN_T, (ncol + TN_T - 1) / TN_T, nsplit);
-  if (prefetch == 2)
-    k_gemm_tn<2><<<grid, 32 * TN_W, 0, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, kchunk, ctas, part);
+  const int al16 = ldw % 2 == 0 && ldx % 2 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)X % 16 == 0;
+  // with dn the kernel follows the bound ncol, as gemm_tn_plan does the count: a
+  // graph bucket lies on one side of kDmmaSmall with every count it serves
+  if (dn) nsplit = gemm_tn_plan_max(M, ncol, K, ctas);
+  if (ncol <= kDmmaSmall)
+    gemm_tn_launch<32, 32, 1, 1, 4, 64, 3>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
+  else if (M > 64)
+    gemm_tn_launch<112, 64, 1, 4, 1, 16, 3>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
   else
-    k_gemm_tn<1><<<grid, 32 * TN_W, 0, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, kchunk, ctas, part);
+    gemm_tn_launch<64, 64, 2, 2, 1, 16, 4>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
 }
 
-__global__ void __launch_bounds__(256) k_gamma_reduce(const double* __restrict__ part, int nsplit, int M,
+// One CTA per column; NG groups of threads share out the splits (then the
+// projectors q of D) of a row r and are summed in a fixed order, so that the
+// loads of a column are in flight together instead of one after the other.
+constexpr int kRedThreads = 512;
+// many columns fill the GPU by themselves and small blocks cost least (1,200
+// columns of 64 projectors: 17 us against 24); few need the width
+static int red_threads(int ncol) { return ncol >= 512 ? 128 : kRedThreads; }
+template <class T, class F>
+WB_DEV void grouped_sum(T* out, T* scratch, int M, int n, F term) {  // out[r] = sum_{i < n} term(r, i)
+  int rw = 32;
+  while (rw < M && rw < (int)blockDim.x) rw *= 2;
+  const int ng = blockDim.x / rw, g = threadIdx.x / rw;
+  for (int r0 = 0; r0 < M; r0 += rw) {
+    const int r = r0 + threadIdx.x % rw;
+    T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+    if (r < M) {
+      int i = g;
+      for (; i + 3 * ng < n; i += 4 * ng) {
+        s0 += term(r, i);
+        s1 += term(r, i + ng);
+        s2 += term(r, i + 2 * ng);
+        s3 += term(r, i + 3 * ng);
+      }
+      for (; i < n; i += ng) s0 += term(r, i);
+    }
+    scratch[threadIdx.x] = (s0 + s1) + (s2 + s3);
+    __syncthreads();
+    if (g == 0 && r < M) {
+      T t = 0;
+      for (int q = 0; q < ng; ++q) t += scratch[q * rw + threadIdx.x];
+      out[r] = t;
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kRedThreads) k_gamma_reduce(const double* __restrict__ part, int nsplit, int M,
                                                       int ncol_host, const int* dn, const double* __restrict__ W,
                                                       long ldw, const double* __restrict__ X, long ldx,
                                                       const int* __restrict__ cols, const double* __restrict__ D,
                                                       int nkb, double alpha, double* __restrict__ C, int K,
                                                       int ctas) {
   extern __shared__ double S[];
+  __shared__ double scratch[kRedThreads];
   const int ncol = dev_count(dn, ncol_host);
   const int j = blockIdx.x;
   if (j >= ncol) return;
-  if (dn && ctas > 0) nsplit = gemm_tn_splits(M, ncol, K, ctas);
+  if (dn && ctas > 0) nsplit = gemm_tn_plan(M, ncol, K, ctas);
   const int col = cols ? cols[j] : j;
   const double x0 = X[(long)col * ldx];
-  for (int r = threadIdx.x; r < M; r += blockDim.x) {
-    double s = 0.0;
-    for (int sp = 0; sp < nsplit; ++sp) s += part[((long)sp * ncol + j) * M + r];
-    S[r] = 2.0 * s - W[(long)r * ldw] * x0;
-  }
+  const double* pj = part + (long)j * M;
+  const long step = (long)ncol * M;
+  grouped_sum(S, scratch, M, nsplit, [&](int r, int i) { return pj[i * step + r]; });
+  for (int r = threadIdx.x; r < M; r += blockDim.x) S[r] = 2.0 * S[r] - W[(long)r * ldw] * x0;
   __syncthreads();
-  for (int r = threadIdx.x; r < M; r += blockDim.x) {
-    double c;
-    if (r < nkb) {
-      c = 0.0;
-      for (int q = 0; q < nkb; ++q) c = fma(D[r + (long)q * nkb], S[q], c);
-    } else {
-      c = alpha * S[r];
-    }
-    C[(long)j * M + r] = c;
-  }
+  double* c = C + (long)j * M;
+  if (nkb > 0) grouped_sum(c, scratch, nkb, nkb, [&](int r, int q) { return D[r + (long)q * nkb] * S[q]; });
+  for (int r = nkb + threadIdx.x; r < M; r += blockDim.x) c[r] = alpha * S[r];
 }
 
 void gamma_reduce(const double* part, int nsplit, int M, int ncol, const double* W, long ldw, const double* X,
                   long ldx, const int* cols, const double* D, int nkb, double alpha, double* C, cudaStream_t s,
                   const int* dn, int K, int ctas) {
   if (ncol <= 0 || M <= 0) return;
-  k_gamma_reduce<<<ncol, 256, sizeof(double) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb,
+  k_gamma_reduce<<<ncol, red_threads(ncol), sizeof(double) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb,
                                                         alpha, C, K, ctas);
 }
 
 // ---------------------------------------------------------------------------
 // Y[col j][k] = beta Y[col j][k] + sum_r W[r][k] C[j][r]
-// CTA: 4 warps x 32 rows of k, 32 columns j; inner loop over r in steps of 4.
-// With beta != 0 (and 16-byte aligned rows of Y) the CTA's Y tile is copied
-// into shared memory by cp.async at the start, so its DRAM latency overlaps
-// the MMAs instead of stalling the epilogue.  Row stride 130 doubles: the four
-// column groups of a half-warp's epilogue reads fall on disjoint banks.
+// CTA: 4 warps x 32 k, 32 columns j; stages of 16 projectors r of W and C stream
+// through a ring of three buffers by cp.async.  With beta != 0 a thread loads its
+// share of Y into registers before the ring starts, so that those reads are in
+// flight during the whole product and the epilogue only adds.  Row strides 132
+// and 20: the fragments of a half-warp fall on distinct banks.
 // ---------------------------------------------------------------------------
-constexpr int NN_YLD = 130;
+constexpr int NN_R = 16, NN_ST = 3, NN_WLD = 132, NN_CLD = 20;
+constexpr int NN_STAGE = NN_R * NN_WLD + 32 * NN_CLD;
 
-WB_DEV void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-
-__global__ void __launch_bounds__(128) k_gemm_nn(const double* __restrict__ W, long ldw, int M,
+__global__ void __launch_bounds__(128, 3) k_gemm_nn(const double* __restrict__ W, long ldw, int M,
                                                  const double* __restrict__ C, double* __restrict__ Y, long ldy,
                                                  const int* __restrict__ cols, int ncol_host, const int* dn, int K,
-                                                 double beta, int stage_y) {
-  __shared__ __align__(16) double ysh[32 * NN_YLD];
+                                                 double beta, int al16) {
+  extern __shared__ __align__(16) double nn_sm[];
   const int ncol = dev_count(dn, ncol_host);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lr = lane >> 2, lk = lane & 3;
-  const int kbase = blockIdx.x * 128;
-  const int k0 = kbase + warp * 32, j0 = blockIdx.y * 32;
+  const int kbase = blockIdx.x * 128, j0 = blockIdx.y * 32;
   if (j0 >= ncol) return;
-  const bool pre = stage_y && beta != 0.0;
-  if (pre) {  // Y[col(j0 + jl)][kbase + 2q, +1] -> ysh[jl][2q, +1]  (K is even: a pair never straddles K)
-    for (int e = threadIdx.x; e < 32 * 64; e += 128) {
-      const int jl = e >> 6, q = e & 63;
-      const int j = j0 + jl, k = kbase + 2 * q;
-      if (j < ncol && k < K) {
-        const int col = cols ? cols[j] : j;
-        cp_async16(ysh + jl * NN_YLD + 2 * q, Y + (long)col * ldy + k);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  }
-  bool kok[4], jok[4];
-  const double* crow[4];
+  auto fetch = [&](int st, int rb) {
+    double* sw = nn_sm + st * NN_STAGE;
+    double* sc = sw + NN_R * NN_WLD;
+    const int kp = (tid & 63) * 2, k = kbase + kp;  // K is even: a pair never straddles it
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    kok[i] = (k0 + i * 8 + lr) < K;
-    const int j = j0 + i * 8 + lr;
-    jok[i] = j < ncol;
-    crow[i] = C + (long)(jok[i] ? j : 0) * M;
+    for (int i = 0; i < NN_R / 2; ++i) {
+      const int rr = (tid >> 6) + 2 * i, r = rb + rr;
+      const bool ok = r < M && k < K;
+      cp_pair(sw + rr * NN_WLD + kp, W + (ok ? (long)r * ldw + k : 0), ok, al16 != 0);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rr = tid & 15, jl = (tid >> 4) + 8 * i, r = rb + rr, j = j0 + jl;
+      const bool ok = r < M && j < ncol;
+      cp_one(sc + jl * NN_CLD + rr, C + (ok ? (long)j * M + r : 0), ok);
+    }
+  };
+#pragma unroll
+  for (int st = 0; st < NN_ST - 1; ++st) {
+    if (st * NN_R < M) fetch(st, st * NN_R);
+    cp_commit();
   }
+  const int k0 = kbase + warp * 32 + lr;
+  double y[4][4][2];
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = j0 + b * 8 + 2 * lk + h;
+      const bool jok = beta != 0.0 && j < ncol;
+      const double* yc = Y + (jok ? (long)(cols ? cols[j] : j) * ldy : 0);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) y[a][b][h] = jok && k0 + a * 8 < K ? yc[k0 + a * 8] : 0.0;
+    }
   double acc[4][4][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-#pragma unroll 4
-  for (int r = 0; r < M; r += 4) {
-    const int rr = r + lk;
-    const bool rok = rr < M;
-    const double* wr = W + (long)(rok ? rr : 0) * ldw + k0 + lr;
-    double av[4], bv[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      av[i] = (rok && kok[i]) ? __ldg(wr + i * 8) : 0.0;
-      bv[i] = (rok && jok[i]) ? __ldg(crow[i] + rr) : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
-  }
-  if (pre) {
-    asm volatile("cp.async.wait_all;\n" ::);
+  int st = 0;
+  for (int rb = 0; rb < M; rb += NN_R) {
+    cp_wait<NN_ST - 2>();
     __syncthreads();
+    const int rn = rb + (NN_ST - 1) * NN_R;
+    if (rn < M) fetch(st == 0 ? NN_ST - 1 : st - 1, rn);
+    cp_commit();
+    const double* sw = nn_sm + st * NN_STAGE + lk * NN_WLD + warp * 32 + lr;
+    const double* sc = nn_sm + st * NN_STAGE + NN_R * NN_WLD + lr * NN_CLD + lk;
+#pragma unroll
+    for (int r = 0; r < NN_R; r += 4) {
+      if (rb + r >= M) break;
+      double av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        av[i] = sw[r * NN_WLD + i * 8];
+        bv[i] = sc[i * 8 * NN_CLD + r];
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
+    }
+    st = st == NN_ST - 1 ? 0 : st + 1;
   }
+  cp_wait<0>();
 #pragma unroll
   for (int b = 0; b < 4; ++b)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int jl = b * 8 + 2 * lk + h, j = j0 + jl;
+      const int j = j0 + b * 8 + 2 * lk + h;
       if (j >= ncol) continue;
-      const int col = cols ? cols[j] : j;
-      double* y = Y + (long)col * ldy;
+      double* yc = Y + (long)(cols ? cols[j] : j) * ldy;
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int kl = warp * 32 + a * 8 + lr, k = kbase + kl;
-        if (k >= K) continue;
-        const double old = beta == 0.0 ? 0.0 : (pre ? ysh[jl * NN_YLD + kl] : y[k]);
-        y[k] = beta * old + acc[a][b][h];
-      }
+      for (int a = 0; a < 4; ++a)
+        if (k0 + a * 8 < K) yc[k0 + a * 8] = beta * y[a][b][h] + acc[a][b][h];
     }
 }
 
 void gemm_nn(const double* W, long ldw, int M, const double* C, double* Y, long ldy, const int* cols, int ncol,
              int K, double beta, cudaStream_t s, const int* dn) {
   if (ncol <= 0 || M <= 0) return;
-  const int stage_y = (K % 2 == 0) && (ldy % 2 == 0) && ((uintptr_t)Y % 16 == 0);
+  const int al16 = ldw % 2 == 0 && (uintptr_t)W % 16 == 0;
+  constexpr int SM = (int)sizeof(double) * NN_STAGE * NN_ST;
   dim3 grid((K + 127) / 128, (ncol + 31) / 32);
-  k_gemm_nn<<<grid, 128, 0, s>>>(W, ldw, M, C, Y, ldy, cols, ncol, dn, K, beta, stage_y);
+  k_gemm_nn<<<grid, 128, SM, s>>>(W, ldw, M, C, Y, ldy, cols, ncol, dn, K, beta, al16);
+}
+
+void la_setup() {
+  cudaFuncSetAttribute(k_gemm_tn<32, 32, 1, 1, 4, 64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       TnTile<32, 32, 1, 1, 4, 64, 3>::SMEM);
+  cudaFuncSetAttribute(k_gemm_tn<64, 64, 2, 2, 1, 16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       TnTile<64, 64, 2, 2, 1, 16, 4>::SMEM);
+  cudaFuncSetAttribute(k_gemm_tn<112, 64, 1, 4, 1, 16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       TnTile<112, 64, 1, 4, 1, 16, 3>::SMEM);
+  cudaFuncSetAttribute(k_gemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(double) * NN_STAGE * NN_ST);
 }
 
 // ---------------------------------------------------------------------------
@@ -495,43 +648,37 @@ void cg_prec_rho32(const int* act, int nact, const float2* g, float2* P, const d
 }
 
 // Active list in increasing system order (map_lbnd2ibnd, :356-382) and the
-// Gamma FFT pairs (act[2k], act[2k+1]).
-__global__ void __launch_bounds__(1024) k_cg_compact(const unsigned char* __restrict__ conv, int nsys_host,
-                                                     const int* nsys_dev, int* __restrict__ act,
-                                                     int2* __restrict__ items, int* __restrict__ nact_out) {
-  const int nsys = dev_count(nsys_dev, nsys_host);
-  __shared__ int wsum[32];
-  __shared__ int base;
+// Gamma FFT pairs (act[2k], act[2k+1]); one block of NT threads.  Returns the
+// count in every thread.
+template <int NT>
+WB_DEV int compact_block(const unsigned char* conv, int nsys, int* act, int2* items, int* nact_out) {
+  __shared__ int wsum[NT / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (tid == 0) base = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < nsys; c0 += 1024) {
+  int base = 0;
+  for (int c0 = 0; c0 < nsys; c0 += NT) {
     const int i = c0 + tid;
-    const bool f = (i < nsys) && !conv[i];
+    const bool f = (i < nsys) && !__ldcg(conv + i);
     const unsigned bal = __ballot_sync(0xffffffffu, f);
-    const int pre = __popc(bal & ((1u << lane) - 1u));
     if (lane == 0) wsum[w] = __popc(bal);
     __syncthreads();
-    if (w == 0) {
-      int v = wsum[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-      }
-      wsum[lane] = v;  // inclusive
+    int off = base, all = base;
+    for (int q = 0; q < NT / 32; ++q) {
+      if (q < w) off += wsum[q];
+      all += wsum[q];
     }
-    __syncthreads();
-    const int off = base + (w > 0 ? wsum[w - 1] : 0) + pre;
-    if (f) act[off] = i;
-    __syncthreads();
-    if (tid == 0) base += wsum[31];
+    if (f) act[off + __popc(bal & ((1u << lane) - 1u))] = i;
+    base = all;
     __syncthreads();
   }
-  const int n = base;
-  for (int k = tid; k < (n + 1) / 2; k += 1024)
-    items[k] = make_int2(act[2 * k], (2 * k + 1 < n) ? act[2 * k + 1] : -1);
-  if (tid == 0) *nact_out = n;
+  for (int k = tid; k < (base + 1) / 2; k += NT)
+    items[k] = make_int2(act[2 * k], (2 * k + 1 < base) ? act[2 * k + 1] : -1);
+  if (tid == 0) *nact_out = base;
+  return base;
+}
+__global__ void __launch_bounds__(1024) k_cg_compact(const unsigned char* __restrict__ conv, int nsys_host,
+                                                     const int* nsys_dev, int* act, int2* __restrict__ items,
+                                                     int* __restrict__ nact_out) {
+  compact_block<1024>(conv, dev_count(nsys_dev, nsys_host), act, items, nact_out);
 }
 void cg_compact(const unsigned char* conv, int nsys, int* act, int2* items, int* nact_dev, int* nact_host,
                 cudaStream_t s, const int* nsys_dev) {
@@ -540,36 +687,114 @@ void cg_compact(const unsigned char* conv, int nsys, int* act, int2* items, int*
 }
 
 
+// End of one PCG pass of the graph-captured loop, by the last CTA of the step
+// kernel to finish: the active list of the next pass and, with ctl, the pass's
+// counters and the loop test of k_loop_bucket and k_loop_ctl (a loop of one
+// bucket needs no kernel of its own for either).
+struct CgTail {
+  int* ticket = nullptr;  // null: no tail; zero between launches
+  const int* nsys = nullptr;
+  int* act = nullptr;
+  int2* items = nullptr;
+  int* nact = nullptr;
+  int* st = nullptr;
+  cudaGraphConditionalHandle cond = 0;
+  int ctl = 0, inner = 0;
+};
+
+WB_DEV void loop_count(int* st, int n) {
+  if (n <= 0) return;
+  *reinterpret_cast<long long*>(st + 4) += n;
+  *reinterpret_cast<long long*>(st + 6) += 2 * ((n + 1) / 2);
+  st[3] += 1;
+}
+WB_DEV void loop_test(cudaGraphConditionalHandle h, int n, int* st, int maxiter, int inner) {
+  const int it = st[1];
+  const bool more = n > 0 && it < maxiter;
+  if (!inner && !more) st[2] = st[3] + (n == 0 ? 1 : 0);
+  if (more) st[1] = it + 1;
+  cudaGraphSetConditional(h, more ? 1u : 0u);
+}
+
+// Two sums over the block, then over the cluster's CTAs in rank order: the same
+// bits in every thread of every CTA.  cl: [2][2] shared slots, used in turn (a
+// CTA is never two reductions ahead of one that still reads).
+template <int NT, int CS>
+WB_DEV double2 cluster_sum2(double a, double b, double* red, double* cl, int& turn) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  constexpr int NW = NT / 32;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __syncthreads();
+  if (l == 0) { red[2 * w] = a; red[2 * w + 1] = b; }
+  __syncthreads();
+  a = l < NW ? red[2 * l] : 0.0;
+  b = l < NW ? red[2 * l + 1] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if constexpr (CS > 1) {
+    double* slot = cl + 2 * turn;
+    turn ^= 1;
+    if (threadIdx.x == 0) { slot[0] = a; slot[1] = b; }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    const unsigned mine = (unsigned)__cvta_generic_to_shared(slot);
+    a = b = 0.0;
+#pragma unroll
+    for (int r = 0; r < CS; ++r) {
+      unsigned peer;
+      double pa, pb;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(r));
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(pa) : "r"(peer) : "memory");
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(pb) : "r"(peer + 8) : "memory");
+      a += pa;
+      b += pb;
+    }
+  }
+  return make_double2(a, b);
+}
+
 // One PCG step after the operator, in one kernel: the update of iteration
 // `iter` (a = <P|g>, c = <P|T> with the Gamma dot, x -= a/c P, g -= a/c T;
 // linsolve_sternheimer_m_wfcts.f90:253-329) and, unless iter == maxiter,
 // iteration iter + 1's preconditioning, rho, test and direction (as
 // k_cg_prec_rho: h = M g, rho = <h|g>, P = -h + rho/rho_prev P).
-// One CTA per system; the new g is preconditioned and its rho summed in the
-// update's own pass, and the direction pass re-reads g (just written) and P
-// (read twice already) from L2, so the vectors make fewer trips to DRAM than
-// with two kernels with the active-list compaction between them.
-template <class C, int NT>
-__global__ void __launch_bounds__(NT) k_cg_step(const int* __restrict__ act, const int* dn, int nhost,
+// One cluster of CS CTAs per system, each with its slice of the plane waves; the
+// new g is preconditioned and its rho summed in the update's own pass, and the
+// later passes re-read P, T and g (just written) from L1 and L2.
+template <class C, int NT, int CS>
+__global__ void __launch_bounds__(NT) k_cg_step(const int* act, const int* dn, int nhost,
                                                 C* __restrict__ x, C* __restrict__ g, C* __restrict__ P,
                                                 const C* __restrict__ T, const double* __restrict__ iprec, int nocc,
                                                 double* rho_prev, unsigned char* conv, int iter_host,
                                                 const int* iter_dev, int maxiter, double tr2,
-                                                const double* __restrict__ rel, double floor, int npw, long ld) {
+                                                const double* __restrict__ rel, double floor, int npw, long ld,
+                                                CgTail tail) {
   using R = real_t<C>;
   __shared__ double red[NT / 16];
+  __shared__ double cl[4];
+  __shared__ int last;
   const int n = dev_count(dn, nhost);
   const int iter = iter_dev ? *iter_dev : iter_host;
   const bool prec = iter + 1 <= maxiter;  // the reference leaves its loop before this preconditioning otherwise
-  for (int b = blockIdx.x; b < n; b += gridDim.x) {
+  const int rank = CS > 1 ? (int)blockIdx.x % CS : 0;
+  const int slice = (npw + CS - 1) / CS, lo = rank * slice, hi = min(npw, lo + slice);
+  int turn = 0;
+  for (int b = blockIdx.x / CS; b < n; b += gridDim.x / CS) {
     const int j = act[b];
     const C* tj = T + (long)j * ld;
     C* pj = P + (long)j * ld;
     C* gj = g + (long)j * ld;
     C* xj = x + (long)j * ld;
     const double* ip = iprec + (long)(j % nocc) * npw;
+    const double rho_last = rho_prev[j];  // read before the reductions, after which rank 0 rewrites it
     double a = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < npw; i += NT) {
+    for (int i = lo + threadIdx.x; i < hi; i += NT) {
       const C p = pj[i], gv = gj[i], tv = tj[i];
       double da = fma((double)p.x, (double)gv.x, (double)p.y * (double)gv.y);
       double dc = fma((double)p.x, (double)tv.x, (double)p.y * (double)tv.y);
@@ -577,10 +802,10 @@ __global__ void __launch_bounds__(NT) k_cg_step(const int* __restrict__ act, con
       a += da;
       c += dc;
     }
-    const double2 s = block_sum2<NT>(a, c, red);
+    const double2 s = cluster_sum2<NT, CS>(a, c, red, cl, turn);
     const R r = R((2.0 * s.x) / (2.0 * s.y));
     double tt = 0.0, t0 = 0.0;
-    for (int i = threadIdx.x; i < npw; i += NT) {
+    for (int i = lo + threadIdx.x; i < hi; i += NT) {
       const C p = pj[i], tv = tj[i];
       const C xv = xj[i], gv = gj[i];
       xj[i] = mkc<C>(fma(-r, p.x, xv.x), fma(-r, p.y, xv.y));
@@ -594,55 +819,118 @@ __global__ void __launch_bounds__(NT) k_cg_step(const int* __restrict__ act, con
       }
     }
     if (!prec) continue;
-    const double2 s2 = block_sum2<NT>(tt, t0, red);
+    const double2 s2 = cluster_sum2<NT, CS>(tt, t0, red, cl, turn);
     const double rho = 2.0 * s2.x - s2.y;
     const double thr = rel ? fmax(tr2 * rel[j], floor) : tr2;
-    if (rho < thr) {  // block-uniform
-      if (threadIdx.x == 0) conv[j] = 1;
+    if (rho < thr) {  // cluster-uniform
+      if (rank == 0 && threadIdx.x == 0) conv[j] = 1;
       continue;
     }
-    const double beta = rho / rho_prev[j];  // iteration iter + 1 >= 2
-    __syncthreads();
-    if (threadIdx.x == 0) rho_prev[j] = rho;
-    for (int i = threadIdx.x; i < npw; i += NT) {
+    const double beta = rho / rho_last;  // iteration iter + 1 >= 2
+    if (rank == 0 && threadIdx.x == 0) rho_prev[j] = rho;
+    for (int i = lo + threadIdx.x; i < hi; i += NT) {
       const double w = ip[i];
       const C gv = gj[i], pv = pj[i];
       const double hx = (double)gv.x * w, hy = (double)gv.y * w;
       pj[i] = mkc<C>(R(fma(beta, (double)pv.x, -hx)), R(fma(beta, (double)pv.y, -hy)));
     }
   }
+  if constexpr (CS > 1)  // no CTA leaves while another of its cluster may read its sums
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (!tail.ticket) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(tail.ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nn = compact_block<NT>(conv, *tail.nsys, tail.act, tail.items, tail.nact);
+  if (threadIdx.x == 0) {
+    *tail.ticket = 0;
+    if (tail.ctl) {
+      loop_count(tail.st, n);
+      loop_test(tail.cond, nn, tail.st, maxiter, tail.inner);
+    }
+  }
 }
 
-// Launch shape of k_cg_step: a persistent grid of a few large CTAs per SM, each
-// looping over systems, so the systems in flight (148 x 540 KB of FP64 vectors,
-// 296 x 270 KB in FP32) keep their vectors in L2 between the kernel's three
-// passes.  With one 256-thread CTA per system (1,200 systems in flight at c2)
-// every pass re-read its vectors from DRAM: 1.22 MB read per FP64 system
-// instead of 0.54 MB (ncu); the FP64 step went from 20.7 to 17.2 ms, the FP32
-// one from 17.2 to 14.8 ms per c2 call.
-static int sm_count() {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) !=
-                                                  cudaSuccess || nsm <= 0)
-      nsm = 148;
-  }
-  return nsm;
+// CTAs per system.  Enough that few systems still cover the SMs (a slice keeps
+// 512 plane waves), and that the systems in flight, one CTA per SM in FP64 and
+// two in FP32, keep their four vectors in L2 between the passes: the 108^3
+// cell's FP64 vectors are 598 KB, 354 MB for 148 systems.  Measured per call
+// there: 4 CTAs 33 ms, 8 41, 1 41 in FP64; 8 CTAs 46 ms, 4 48, 1 68 in FP32; at
+// 64^3 (80 MB for 148 systems) 1 CTA 16.7 ms, 2 20.7.  One perturbation at 64^3,
+// 19 systems: 24 us a step with one CTA each, 13 with 4.
+static int cg_cluster(int nmax, int npw, int elem) {
+  const int ctas = elem == 16 ? sm_count() : 2 * sm_count();
+  int cs = 1;
+  while (cs < 8 && (long)nmax * 2 * cs <= ctas && 2 * cs * 512 <= npw) cs *= 2;
+  while (cs < 8 && 4.0 * elem * npw * (double)std::min(nmax, ctas / cs) > (cs > 1 && elem == 8 ? 50e6 : 96e6)) cs *= 2;
+  return cs;
+}
+template <class C, int NT, int CS, class... A>
+static void cg_step_launch(int nact, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  // one CTA per system: a persistent grid, so that no more systems than fit L2 are in flight
+  const int resident = (sizeof(C) == 16 ? 1 : 2) * sm_count();
+  cfg.gridDim = dim3(CS == 1 ? std::min(nact, resident) : nact * CS);
+  cfg.blockDim = dim3(NT);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_cg_step<C, NT, CS>, args...);
+}
+static CgTail cg_tail(const CgLoop* l) {
+  CgTail t;
+  if (!l) return t;
+  t.ticket = l->st + 8;
+  t.nsys = l->st;
+  t.act = l->act;
+  t.items = l->items;
+  t.nact = l->nact;
+  t.st = l->st;
+  t.cond = l->cond;
+  t.ctl = l->ctl;
+  t.inner = l->inner;
+  return t;
 }
 void cg_step(const int* act, int nact, double2* x, double2* g, double2* P, const double2* T, const double* iprec,
              int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double tr2, int npw, long ld,
-             cudaStream_t s, const int* dn, const int* iter_dev) {
+             cudaStream_t s, const int* dn, const int* iter_dev, const CgLoop* loop) {
   if (nact <= 0) return;
-  k_cg_step<double2, 1024><<<std::min(nact, sm_count()), 1024, 0, s>>>(
-      act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, tr2, nullptr, 0.0, npw, ld);
+  const double* rel = nullptr;
+  auto go = [&](auto launch) {
+    launch(nact, s, act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, tr2, rel, 0.0,
+           npw, ld, cg_tail(loop));
+  };
+  if (npw <= 1024) return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 256, 1>(m, q, a...); });
+  switch (cg_cluster(nact, npw, 16)) {
+    case 1: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 1>(m, q, a...); });
+    case 2: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 2>(m, q, a...); });
+    case 4: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 4>(m, q, a...); });
+    default: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 8>(m, q, a...); });
+  }
 }
 void cg_step32(const int* act, int nact, float2* x, float2* g, float2* P, const float2* T, const double* iprec,
                int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double eta, const double* rel,
-               double floor, int npw, long ld, cudaStream_t s, const int* dn, const int* iter_dev) {
+               double floor, int npw, long ld, cudaStream_t s, const int* dn, const int* iter_dev,
+               const CgLoop* loop) {
   if (nact <= 0) return;
-  k_cg_step<float2, 512><<<std::min(nact, 2 * sm_count()), 512, 0, s>>>(
-      act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, eta, rel, floor, npw, ld);
+  auto go = [&](auto launch) {
+    launch(nact, s, act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, eta, rel, floor,
+           npw, ld, cg_tail(loop));
+  };
+  if (npw <= 1024) return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 256, 1>(m, q, a...); });
+  switch (cg_cluster(nact, npw, 8)) {
+    case 1: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 1>(m, q, a...); });
+    case 2: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 2>(m, q, a...); });
+    case 4: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 4>(m, q, a...); });
+    default: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 8>(m, q, a...); });
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -813,7 +1101,7 @@ void gemm_tn32(const float* W, long ldw, int M, const float* X, long ldx, const 
   k_gemm_tn_f32<<<grid, 256, 0, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, kchunk, part);
 }
 
-__global__ void __launch_bounds__(256) k_gamma_reduce32(const float* __restrict__ part, int nsplit, int M,
+__global__ void __launch_bounds__(kRedThreads) k_gamma_reduce32(const float* __restrict__ part, int nsplit, int M,
                                                         int ncol_host, const int* dn,
                                                         const float* __restrict__ W, long ldw,
                                                         const float* __restrict__ X, long ldx,
@@ -821,6 +1109,7 @@ __global__ void __launch_bounds__(256) k_gamma_reduce32(const float* __restrict_
                                                         int nkb, float alpha, float* __restrict__ C, int K,
                                                         int umma_ctas) {
   extern __shared__ float Sf[];
+  __shared__ float scratch[kRedThreads];
   const int ncol = dev_count(dn, ncol_host);
   const int j = blockIdx.x;
   if (j >= ncol) return;
@@ -830,28 +1119,20 @@ __global__ void __launch_bounds__(256) k_gamma_reduce32(const float* __restrict_
   }
   const int col = cols ? cols[j] : j;
   const float x0 = X[(long)col * ldx];
-  for (int r = threadIdx.x; r < M; r += blockDim.x) {
-    float sum = 0.f;
-    for (int sp = 0; sp < nsplit; ++sp) sum += part[((long)sp * ncol + j) * M + r];
-    Sf[r] = 2.f * sum - W[(long)r * ldw] * x0;
-  }
+  const float* pj = part + (long)j * M;
+  const long step = (long)ncol * M;
+  grouped_sum(Sf, scratch, M, nsplit, [&](int r, int i) { return pj[i * step + r]; });
+  for (int r = threadIdx.x; r < M; r += blockDim.x) Sf[r] = 2.f * Sf[r] - W[(long)r * ldw] * x0;
   __syncthreads();
-  for (int r = threadIdx.x; r < M; r += blockDim.x) {
-    float c;
-    if (r < nkb) {
-      c = 0.f;
-      for (int q = 0; q < nkb; ++q) c = fmaf(D[r + (long)q * nkb], Sf[q], c);
-    } else {
-      c = alpha * Sf[r];
-    }
-    C[(long)j * M + r] = c;
-  }
+  float* c = C + (long)j * M;
+  if (nkb > 0) grouped_sum(c, scratch, nkb, nkb, [&](int r, int q) { return D[r + (long)q * nkb] * Sf[q]; });
+  for (int r = nkb + threadIdx.x; r < M; r += blockDim.x) c[r] = alpha * Sf[r];
 }
 void gamma_reduce32(const float* part, int nsplit, int M, int ncol, const float* W, long ldw, const float* X, long ldx,
                     const int* cols, const float* D, int nkb, float alpha, float* C, cudaStream_t s, const int* dn,
                     int K, int umma_ctas) {
   if (ncol <= 0 || M <= 0) return;
-  k_gamma_reduce32<<<ncol, 256, sizeof(float) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb, alpha,
+  k_gamma_reduce32<<<ncol, red_threads(ncol), sizeof(float) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb, alpha,
                                                         C, K, umma_ctas);
 }
 
@@ -918,11 +1199,13 @@ void gemm_nn32_acc(const float* W, long ldw, int M, const float* C, float* Y, lo
 // ---------------------------------------------------------------------------
 // st[0] systems of the batch, st[1] iteration of the next pass, st[2] last
 // iteration run, st[3] inner iterations run over all refinements (mixed form);
-// st[4..5] active system-iterations and st[6..7] FFT boxes (64-bit counters).
+// st[4..5] active system-iterations and st[6..7] FFT boxes (64-bit counters);
+// st[8] ticket of the step kernel's last CTA (zero between launches).
 __global__ void k_loop_init(int* st, int nsys, int reset_totals) {
   st[0] = nsys;
   st[1] = 1;
   st[2] = 0;
+  st[8] = 0;
   if (reset_totals) {
     st[3] = 0;
     *reinterpret_cast<long long*>(st + 4) = 0;
@@ -942,11 +1225,7 @@ void loop_init(int* st, int nsys, bool reset_totals, cudaStream_t s) {
 // count in st[2]: the passes that did work, plus the one whose test found no
 // system left.
 __global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int* nact, int* st, int maxiter, int inner) {
-  const int n = *nact, it = st[1];
-  const bool more = n > 0 && it < maxiter;
-  if (!inner && !more) st[2] = st[3] + (n == 0 ? 1 : 0);
-  if (more) st[1] = it + 1;
-  cudaGraphSetConditional(h, more ? 1u : 0u);
+  loop_test(h, *nact, st, maxiter, inner);
 }
 void loop_ctl(cudaGraphConditionalHandle h, const int* nact, int* st, int maxiter, bool inner, cudaStream_t s) {
   k_loop_ctl<<<1, 1, 0, s>>>(h, nact, st, maxiter, inner ? 1 : 0);
@@ -958,11 +1237,7 @@ void loop_ctl(cudaGraphConditionalHandle h, const int* nact, int* st, int maxite
 // bucket: the workspace capacity).
 __global__ void k_loop_bucket(cudaGraphConditionalHandle h, const int* nact, int* st, int min_items, int nbuckets) {
   const int n = *nact;
-  if (n > 0) {
-    *reinterpret_cast<long long*>(st + 4) += n;
-    *reinterpret_cast<long long*>(st + 6) += 2 * ((n + 1) / 2);
-    st[3] += 1;
-  }
+  loop_count(st, n);
   const int items = (n + 1) / 2;
   int k = 0;
   while (k < nbuckets - 1 && (min_items << k) < items) ++k;
