@@ -152,6 +152,7 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
   c->st.cmap = c->cmap.as<int>();
   c->st.prune = prune;
   if (rt) {
+    if (ncols < 2) c->geo.fast = nullptr;  // RPlane divides by multiplication, which has no 1
     c->geo.colx = c->rt_colx.as<int>();
     c->geo.spos = c->stpos.as<int>();
   }
@@ -1097,6 +1098,7 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
     c->geo.px = rt_plan(s->nr1);
     c->geo.py = rt_plan(s->nr2);
     c->geo.pz = rt_plan(s->nr3);
+    c->geo.fast = rt_fast_setup(s->nr1, s->nr2, &c->rt_fast) ? &c->rt_fast : nullptr;
   }
   c->nocc = s->nbnd_occ;
   c->nkb = s->nkb;
@@ -1152,17 +1154,22 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
     raw.release();
     if (ev != cudaSuccess) return bail(fail(WB_ERR_CUDA, std::string("V(r) layout: ") + cudaGetErrorString(ev)));
   } else {
+    // V(r) / N where the transforms leave real space: z digit-reversed; the
+    // planes digit-reversed too, or [x][ys] (wb_plane.cuh)
     vsc.resize(c->nnr);
-    // V(r) / N at the digit-reversed positions the runtime transforms leave real space in
     const int nx = s->nr1, ny = s->nr2, nz = s->nr3;
+    const bool fast = c->geo.fast != nullptr;
     std::vector<int> rx(nx), ry(ny), rz(nz);
-    for (int p = 0; p < nx; ++p) rx[p] = rt_digit_reverse(c->geo.px, p);
-    for (int p = 0; p < ny; ++p) ry[p] = rt_digit_reverse(c->geo.py, p);
+    for (int p = 0; p < nx; ++p) rx[p] = fast ? p : rt_digit_reverse(c->geo.px, p);
+    for (int p = 0; p < ny; ++p)
+      ry[p] = fast ? p / c->rt_fast.by + c->rt_fast.ay * (p % c->rt_fast.by) : rt_digit_reverse(c->geo.py, p);
     for (int p = 0; p < nz; ++p) rz[p] = rt_digit_reverse(c->geo.pz, p);
     for (int pz = 0; pz < nz; ++pz)
       for (int py = 0; py < ny; ++py)
-        for (int px = 0; px < nx; ++px)
-          vsc[((size_t)pz * ny + py) * nx + px] = s->vrs[((size_t)rz[pz] * ny + ry[py]) * nx + rx[px]] / (double)c->nnr;
+        for (int px = 0; px < nx; ++px) {
+          const size_t to = fast ? ((size_t)pz * nx + px) * ny + py : ((size_t)pz * ny + py) * nx + px;
+          vsc[to] = s->vrs[((size_t)rz[pz] * ny + ry[py]) * nx + rx[px]] / (double)c->nnr;
+        }
     if ((rc = upload(twiddles(nx).data(), nx, c->twx)) || (rc = upload(twiddles(ny).data(), ny, c->twy)) ||
         (rc = upload(twiddles(nz).data(), nz, c->twz)))
       return bail(rc);
@@ -1190,7 +1197,7 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
     if ((rc = upload(dd.data(), dd.size(), c->D))) return bail(rc);
   }
   la_setup();
-  if (c->rt) rt_setup(c->geo);
+  if (c->rt) rt_setup();
   else fft_setup(N);
   c->fa.n = N;
   c->fa.st = c->st;

@@ -58,6 +58,7 @@ struct wb_ctx {
   int nz = 0;                // stick length (box edge along z)
   int rt = 0;                // 1: runtime-size FFT path (no compiled kernels for this box)
   wb::RtGeo geo{};           // its geometry (radix plans, active columns, twiddle tables)
+  wb::RtFast rt_fast;        // its plane phases (geo.fast points here where they apply)
   DBuf rt_colx, twx, twy, twz, twx32, twy32, twz32;
   double omega = 0, wk = 0, alpha = 0;
   wb::StickTab st{};

@@ -14,13 +14,19 @@
 // multiplied point by point with each other and with V(r), which the host
 // stores in the same permuted layout.
 //
-// The x-y pass keeps only the plane's active columns (the x values of the
-// sticks) in shared memory, column-major with an odd column stride; rows are
-// transformed in chunks of full length through a row scratch area.
+// The x-y pass of most boxes (edges a * b with radices up to 16, the full plane
+// in shared memory) runs the phases of wb_plane.cuh with the radices dispatched
+// per phase: 45 x 54 planes take 1.2 us per FP64 item and z-plane set instead of
+// 5.2 with the staged kernels.  The others (125, 128 x 128 in FP64, ...) keep only
+// the plane's active columns (the x values of the sticks) in shared memory,
+// column-major with an odd column stride; rows are transformed in chunks of full
+// length through a row scratch area.
 #include <algorithm>
 
-#include "wb_fft.cuh"
+#include <cmath>
+
 #include "wb_internal.h"
+#include "wb_plane.cuh"
 
 namespace wb {
 
@@ -404,6 +410,200 @@ __global__ void __launch_bounds__(kRtPnt, 1) k_plane_drho_rt(const double2* __re
 }
 
 // ---------------------------------------------------------------------------
+// x-y passes by the phases of wb_plane.cuh, radices dispatched per phase
+// ---------------------------------------------------------------------------
+// The edge's split: both radices in the list, the larger first, as even as
+// possible (fewer points per thread leave more threads per SM).
+static bool rt_radix(int r) {
+  for (int q : {3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16})
+    if (q == r) return true;
+  return false;
+}
+void rt_split(int n, int* a, int* b) {
+  *a = *b = 0;
+  for (int q = 3; q * q <= n; ++q)
+    if (n % q == 0 && rt_radix(q) && rt_radix(n / q)) { *a = n / q; *b = q; }
+}
+static size_t rt_fast_smem(int nx, int ny, size_t elem) { return elem * (size_t)ny * (nx | 1); }
+bool rt_fast_setup(int nx, int ny, RtFast* f) {
+  if (nx > kRtMaxEdge || ny > kRtMaxEdge || rt_fast_smem(nx, ny, 16) > 227u * 1024u) return false;
+  rt_split(nx, &f->ax, &f->bx);
+  rt_split(ny, &f->ay, &f->by);
+  if (!f->ax || !f->ay) return false;
+  f->max_radix = std::max(std::max(f->ax, f->bx), std::max(f->ay, f->by));
+  auto fill = [](int n, int b, double2* t, float2* t32) {
+    for (int i = 0; i < n; ++i) {
+      const long double w = 2.0L * 3.14159265358979323846264338327950288L * (long double)((i / b) * (i % b) % n) / n;
+      t[i] = make_double2((double)cosl(w), (double)sinl(w));
+      t32[i] = make_float2((float)t[i].x, (float)t[i].y);
+    }
+  };
+  fill(nx, f->bx, f->tx, f->tx32);
+  fill(ny, f->by, f->ty, f->ty32);
+  return true;
+}
+
+template <class C>
+struct RtTw {
+  C x[kRtMaxEdge], y[kRtMaxEdge];
+};
+// one dimension's step factors in the constant bank
+template <class C, bool Y>
+struct RtTwOf {
+  const RtTw<C>& t;
+  WB_DEV C operator()(int i) const { return Y ? t.y[i] : t.x[i]; }
+};
+template <int R> struct Radix { static constexpr int value = R; };
+// f(Radix<r>) for the run-time radix r <= MAXR (uniform over the CTA)
+template <int MAXR, class F>
+WB_DEV void with_radix(int r, F f) {
+  switch (r) {
+    case 3: f(Radix<3>{}); break;
+    case 4: f(Radix<4>{}); break;
+    case 5: f(Radix<5>{}); break;
+    case 6: f(Radix<6>{}); break;
+    case 7: f(Radix<7>{}); break;
+    case 8: f(Radix<8>{}); break;
+    case 9: f(Radix<9>{}); break;
+    case 10: f(Radix<10>{}); break;
+    default:
+      if constexpr (MAXR > 10) {
+        if (r == 12) f(Radix<12>{});
+        else if (r == 15) f(Radix<15>{});
+        else f(Radix<16>{});
+      }
+  }
+}
+#define WB_RADIX(r, call) with_radix<MAXR>(r, [&](auto radix_) { constexpr int R = decltype(radix_)::value; call; })
+
+template <int MAXR, class C>
+WB_DEV void rtf_inverse(C* pl, const RtTw<C>& tw, const C* sz, const StickTab& st, const RPlane& g) {
+  const int nt = blockDim.x;
+  const RtTwOf<C, false> tx{tw};
+  const RtTwOf<C, true> ty{tw};
+  WB_RADIX(g.ay_, (plane_col_in<R>(pl, ty, sz, st.cmap, g, nt)));
+  __syncthreads();
+  WB_RADIX(g.by_, (plane_col_mid_inv<R>(pl, g, nt)));
+  __syncthreads();
+  WB_RADIX(g.ax_, (plane_row_in<R>(pl, tx, g, nt)));
+  __syncthreads();
+}
+template <int MAXR, class C>
+WB_DEV void rtf_forward(C* pl, const RtTw<C>& tw, C* sz, const StickTab& st, const RPlane& g) {
+  const int nt = blockDim.x;
+  const RtTwOf<C, true> ty{tw};
+  __syncthreads();
+  WB_RADIX(g.ax_, (plane_row_out<R>(pl, g, nt)));
+  __syncthreads();
+  WB_RADIX(g.by_, (plane_col_mid_fwd<R>(pl, ty, g, nt)));
+  __syncthreads();
+  WB_RADIX(g.ay_, (plane_col_out<R>(pl, sz, st.cmap, g, nt)));
+}
+
+// Two builds of each kernel.  Radices up to 10 and planes of which three or more
+// fit an SM: 80 registers, blocks of 192 threads where four planes fit (45 x 54:
+// 1.24 us per FP64 item against 1.32 with three of 256 and 1.52 with two), else of
+// 256.  The others: 128 registers, two blocks of 256 or one of 512.
+template <int MAXR>
+constexpr int rtf_max_threads() { return MAXR <= 10 ? 256 : 512; }
+template <int MAXR>
+constexpr int rtf_blocks() { return MAXR <= 10 ? 3 : 1; }
+struct RtfShape {
+  bool small;
+  int threads;
+};
+static RtfShape rtf_shape(const RtGeo& g, size_t elem) {
+  const int fit = (int)(227u * 1024u / (rt_fast_smem(g.nx, g.ny, elem) + 1024));
+  const bool small = g.fast->max_radix <= 10 && fit >= 3;
+  return {small, small ? (fit >= 4 ? 192 : 256) : (fit >= 2 ? 256 : 512)};
+}
+
+// psi -> V(r) psi(r) / N -> back, in place on the sticks of plane pz of item
+template <int MAXR, class C>
+__global__ void __launch_bounds__(rtf_max_threads<MAXR>(), rtf_blocks<MAXR>()) k_plane_vloc_rtf(
+    C* __restrict__ sticks, StickTab st, const __grid_constant__ RPlane g, const real_t<C>* __restrict__ vs,
+    const __grid_constant__ RtTw<C> tw, const int* dn) {
+  if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;
+  C* pl = rt_smem<C>();
+  const int nt = blockDim.x;
+  C* sz = sticks + ((long)blockIdx.y * gridDim.x + blockIdx.x) * st.nst;
+  const RtTwOf<C, false> tx{tw};
+  rtf_inverse<MAXR>(pl, tw, sz, st, g);
+  WB_RADIX(g.bx_, (plane_row_vloc<R>(pl, tx, vs + (long)blockIdx.x * g.nx_ * g.ny_, g, nt)));
+  rtf_forward<MAXR>(pl, tw, sz, st, g);
+}
+
+// sticks -> real-space box, no scaling
+template <int MAXR>
+__global__ void __launch_bounds__(rtf_max_threads<MAXR>(), rtf_blocks<MAXR>()) k_plane_inv_box_rtf(
+    const double2* __restrict__ sticks, StickTab st, const __grid_constant__ RPlane g, double2* __restrict__ box,
+    const __grid_constant__ RtTw<double2> tw) {
+  double2* pl = rt_smem<double2>();
+  const long plane = (long)blockIdx.y * gridDim.x + blockIdx.x;
+  rtf_inverse<MAXR>(pl, tw, sticks + plane * st.nst, st, g);
+  WB_RADIX(g.bx_, (plane_row_box<R>(pl, box + plane * g.nx_ * g.ny_, g, (int)blockDim.x)));
+}
+
+// RHS (dfpt_module.f90:245-260), one CTA per (plane, perturbation, band pair)
+template <int MAXR>
+__global__ void __launch_bounds__(rtf_max_threads<MAXR>(), rtf_blocks<MAXR>()) k_plane_rhs_rtf(
+    const double2* __restrict__ evcr, const double2* __restrict__ dvbox, int npv, StickTab st,
+    const __grid_constant__ RPlane g, double2* __restrict__ sticks, const __grid_constant__ RtTw<double2> tw) {
+  double2* pl = rt_smem<double2>();
+  const int pz = blockIdx.x, nz = gridDim.x, p = blockIdx.y, nt = blockDim.x;
+  const long plane = (long)g.nx_ * g.ny_;
+  const double inv = 1.0 / ((double)plane * nz);
+  const double2* dv = dvbox + ((long)(p >> 1) * nz + pz) * plane;
+  const RtTwOf<double2, false> tx{tw};
+  for (int k = 0; k < npv; ++k) {
+    __syncthreads();  // the previous band pair's column pass is done with the plane
+    WB_RADIX(g.bx_, (plane_row_rhs<R>(pl, tx, evcr + ((long)k * nz + pz) * plane, dv, (p & 1) != 0, inv, g, nt)));
+    rtf_forward<MAXR>(pl, tw, sticks + (((long)p * npv + k) * nz + pz) * st.nst, st, g);
+  }
+}
+
+// density response (dfpt_module.f90:403-423, :478) of the perturbations 2 pp and
+// 2 pp + 1, summed over the bands in the CTA's own slice of acc
+template <int MAXR>
+__global__ void __launch_bounds__(rtf_max_threads<MAXR>(), rtf_blocks<MAXR>()) k_plane_drho_rtf(
+    const double2* __restrict__ dsticks, const double2* __restrict__ evcr, const double* __restrict__ occ, int nocc,
+    int mb, StickTab st, const __grid_constant__ RPlane g, double2* __restrict__ acc, double scale,
+    double2* __restrict__ osticks, const __grid_constant__ RtTw<double2> tw) {
+  double2* pl = rt_smem<double2>();
+  const int pz = blockIdx.x, nz = gridDim.x, pp = blockIdx.y, nt = blockDim.x;
+  const int npv = (nocc + 1) / 2;
+  const long plane = (long)g.nx_ * g.ny_;
+  double* sum = reinterpret_cast<double*>(acc + ((long)pp * nz + pz) * plane);
+  const RtTwOf<double2, false> tx{tw};
+  for (int p = 2 * pp; p < min(mb, 2 * pp + 2); ++p)
+    for (int k = 0; k < npv; ++k) {
+      __syncthreads();
+      rtf_inverse<MAXR>(pl, tw, dsticks + (((long)p * npv + k) * nz + pz) * st.nst, st, g);
+      const double o1 = occ[2 * k], o2 = (2 * k + 1 < nocc) ? occ[2 * k + 1] : 0.0;
+      WB_RADIX(g.bx_, (plane_row_density<R>(pl, evcr + ((long)k * nz + pz) * plane, sum + (p & 1) * plane, o1, o2,
+                                            k == 0, g, nt)));
+    }
+  __syncthreads();
+  // an odd batch: the second density of the last pair is zero
+  WB_RADIX(g.bx_, (plane_row_pair<R>(pl, tx, sum, 2 * pp + 1 < mb ? sum + plane : nullptr, scale, g, nt)));
+  rtf_forward<MAXR>(pl, tw, osticks + ((long)pp * nz + pz) * st.nst, st, g);
+}
+
+static RPlane rtf_plane(const RtGeo& g, const StickTab& st) {
+  const RtFast& f = *g.fast;
+  auto magic = [](int d) { return (unsigned)((0x100000000ull + d - 1) / d); };
+  return RPlane{g.nx, g.ny, f.ax, f.bx, f.ay, f.by, st.ncols, st.xhi + 1, magic(st.ncols), magic(g.ny)};
+}
+template <class C>
+static RtTw<C> rtf_tw(const RtGeo& g) {
+  RtTw<C> t;
+  for (int i = 0; i < kRtMaxEdge; ++i) {
+    if constexpr (sizeof(C) == 16) { t.x[i] = g.fast->tx[i]; t.y[i] = g.fast->ty[i]; }
+    else { t.x[i] = g.fast->tx32[i]; t.y[i] = g.fast->ty32[i]; }
+  }
+  return t;
+}
+// ---------------------------------------------------------------------------
 // epilogues of the forward z pass (the same operations as wb_fft_kernels.cu's)
 // ---------------------------------------------------------------------------
 struct RtEpiStore {
@@ -474,20 +674,24 @@ template <class C>
 static size_t rt_zsmem(const RtGeo& g) { return sizeof(C) * (g.nz + 2 * kRtZsg * (g.nz | 1)); }
 static dim3 rt_zgrid(const StickTab& st, int nitems) { return dim3((st.nsp + kRtZsg - 1) / kRtZsg, nitems); }
 
-void rt_setup(const RtGeo& g) {
-  const int z64 = (int)rt_zsmem<double2>(g), z32 = (int)rt_zsmem<float2>(g);
-  const int p64 = (int)rt_plane_smem(g, 16, nullptr), p32 = (int)rt_plane_smem(g, 8, nullptr);
-  cudaFuncSetAttribute(k_zinv_rt<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, z64);
-  cudaFuncSetAttribute(k_zinv_rt<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, z32);
-  cudaFuncSetAttribute(k_zfwd_rt<double2, RtEpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, z64);
-  cudaFuncSetAttribute(k_zfwd_rt<double2, RtEpiHpsi<double2>>, cudaFuncAttributeMaxDynamicSharedMemorySize, z64);
-  cudaFuncSetAttribute(k_zfwd_rt<float2, RtEpiHpsi<float2>>, cudaFuncAttributeMaxDynamicSharedMemorySize, z32);
-  cudaFuncSetAttribute(k_zfwd_rt<double2, RtEpiDng>, cudaFuncAttributeMaxDynamicSharedMemorySize, z64);
-  cudaFuncSetAttribute(k_plane_vloc_rt<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, p64);
-  cudaFuncSetAttribute(k_plane_vloc_rt<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, p32);
-  cudaFuncSetAttribute(k_plane_inv_box_rt, cudaFuncAttributeMaxDynamicSharedMemorySize, p64);
-  cudaFuncSetAttribute(k_plane_rhs_rt, cudaFuncAttributeMaxDynamicSharedMemorySize, p64);
-  cudaFuncSetAttribute(k_plane_drho_rt, cudaFuncAttributeMaxDynamicSharedMemorySize, p64);
+// The kernels serve contexts of several boxes, so each is opted in to all the
+// shared memory a CTA can have rather than to one box's size.
+constexpr int kRtMaxSmem = 227 * 1024;
+template <class... K>
+static void opt_in(K*... k) {
+  (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kRtMaxSmem), ...);
+}
+template <int MAXR>
+static void rtf_setup() {
+  opt_in(k_plane_vloc_rtf<MAXR, double2>, k_plane_vloc_rtf<MAXR, float2>, k_plane_inv_box_rtf<MAXR>,
+         k_plane_rhs_rtf<MAXR>, k_plane_drho_rtf<MAXR>);
+}
+void rt_setup() {
+  opt_in(k_zinv_rt<double2>, k_zinv_rt<float2>, k_zfwd_rt<double2, RtEpiStore>, k_zfwd_rt<double2, RtEpiHpsi<double2>>,
+         k_zfwd_rt<float2, RtEpiHpsi<float2>>, k_zfwd_rt<double2, RtEpiDng>, k_plane_vloc_rt<double2>,
+         k_plane_vloc_rt<float2>, k_plane_inv_box_rt, k_plane_rhs_rt, k_plane_drho_rt);
+  rtf_setup<10>();
+  rtf_setup<16>();
 }
 
 template <class C, class F>
@@ -505,6 +709,13 @@ static void zfwd_rt_t(const F& f, const C* sticks, const int2* items, int nitems
 template <class C, class F>
 static void vloc_rt_t(const F& f, C* sticks, int nitems, const real_t<C>* vs) {
   if (nitems <= 0) return;
+  if (f.rt->fast) {
+    const RtfShape sh = rtf_shape(*f.rt, sizeof(C));
+    auto k = sh.small ? k_plane_vloc_rtf<10, C> : k_plane_vloc_rtf<16, C>;
+    k<<<dim3(f.rt->nz, nitems), sh.threads, rt_fast_smem(f.rt->nx, f.rt->ny, sizeof(C)), f.stream>>>(
+        sticks, f.st, rtf_plane(*f.rt, f.st), vs, rtf_tw<C>(*f.rt), f.dcount);
+    return;
+  }
   int rc = 1;
   const size_t sm = rt_plane_smem(*f.rt, sizeof(C), &rc);
   k_plane_vloc_rt<C><<<dim3(f.rt->nz, nitems), kRtPnt, sm, f.stream>>>(sticks, f.st, *f.rt, vs, rc, f.dcount);
@@ -539,12 +750,26 @@ void rt_plane_vloc32(const FftArgs32& f, float2* sticks, int nitems, const float
 }
 void rt_plane_inv_box(const FftArgs& f, const double2* sticks, int nitems, double2* box) {
   if (nitems <= 0) return;
+  if (f.rt->fast) {
+    const RtfShape sh = rtf_shape(*f.rt, 16);
+    auto k = sh.small ? k_plane_inv_box_rtf<10> : k_plane_inv_box_rtf<16>;
+    k<<<dim3(f.rt->nz, nitems), sh.threads, rt_fast_smem(f.rt->nx, f.rt->ny, 16), f.stream>>>(
+        sticks, f.st, rtf_plane(*f.rt, f.st), box, rtf_tw<double2>(*f.rt));
+    return;
+  }
   int rc = 1;
   const size_t sm = rt_plane_smem(*f.rt, 16, &rc);
   k_plane_inv_box_rt<<<dim3(f.rt->nz, nitems), kRtPnt, sm, f.stream>>>(sticks, f.st, *f.rt, box, rc);
 }
 void rt_plane_rhs(const FftArgs& f, const double2* evcr, const double2* dvbox, int npv, int mb, double2* sticks) {
   if (mb <= 0) return;
+  if (f.rt->fast) {
+    const RtfShape sh = rtf_shape(*f.rt, 16);
+    auto k = sh.small ? k_plane_rhs_rtf<10> : k_plane_rhs_rtf<16>;
+    k<<<dim3(f.rt->nz, mb), sh.threads, rt_fast_smem(f.rt->nx, f.rt->ny, 16), f.stream>>>(
+        evcr, dvbox, npv, f.st, rtf_plane(*f.rt, f.st), sticks, rtf_tw<double2>(*f.rt));
+    return;
+  }
   int rc = 1;
   const size_t sm = rt_plane_smem(*f.rt, 16, &rc);
   k_plane_rhs_rt<<<dim3(f.rt->nz, mb), kRtPnt, sm, f.stream>>>(evcr, dvbox, npv, f.st, *f.rt, sticks, rc);
@@ -552,6 +777,13 @@ void rt_plane_rhs(const FftArgs& f, const double2* evcr, const double2* dvbox, i
 void rt_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evcr, const double* occ, int nocc,
                    int mb, double2* acc, double scale, double2* osticks) {
   if (mb <= 0) return;
+  if (f.rt->fast) {
+    const RtfShape sh = rtf_shape(*f.rt, 16);
+    auto k = sh.small ? k_plane_drho_rtf<10> : k_plane_drho_rtf<16>;
+    k<<<dim3(f.rt->nz, (mb + 1) / 2), sh.threads, rt_fast_smem(f.rt->nx, f.rt->ny, 16), f.stream>>>(
+        dsticks, evcr, occ, nocc, mb, f.st, rtf_plane(*f.rt, f.st), acc, scale, osticks, rtf_tw<double2>(*f.rt));
+    return;
+  }
   int rc = 1;
   const size_t sm = rt_plane_smem(*f.rt, 16, &rc);
   k_plane_drho_rt<<<dim3(f.rt->nz, (mb + 1) / 2), kRtPnt, sm, f.stream>>>(dsticks, evcr, occ, nocc, mb, f.st,

@@ -27,6 +27,17 @@ struct StickTab {
 // (digit-reversed input, natural output).  Real-space data therefore sit at
 // digit-reversed positions in every direction; they are only ever multiplied
 // point by point, with V(r) stored in the same permuted layout.
+// Boxes whose x and y edges split as a * b with radices up to 16 and whose full
+// plane fits in shared memory run the plane phases of wb_plane.cuh instead, with
+// the splits and twiddles below taken at run time (real space is then [pz][x][ys]).
+constexpr int kRtMaxEdge = 160;
+struct RtFast {
+  int ax = 0, bx = 0, ay = 0, by = 0, max_radix = 0;
+  double2 tx[kRtMaxEdge], ty[kRtMaxEdge];  // W_n^(k1 n2) at k1 b + n2
+  float2 tx32[kRtMaxEdge], ty32[kRtMaxEdge];
+};
+// the split of an edge (0, 0 if it has none)
+void rt_split(int n, int* a, int* b);
 constexpr int kRtMaxStages = 16;
 struct RtPlan {
   int n, ns;
@@ -41,11 +52,14 @@ struct RtGeo {
   const int* spos;           // [nst] half-plane offset c * cs + (y mod ny) of each stick, -1 = dummy
   const double2 *twx, *twy, *twz;  // exp(+2 pi i j / n) per direction
   const float2 *twx32, *twy32, *twz32;
+  const RtFast* fast;        // host pointer; null: the staged kernels
 };
 // radix stages of n (empty if n has a prime factor above 7)
 RtPlan rt_plan(int n);
 // box index in a direction of the value stored at position p by the inverse
 int rt_digit_reverse(const RtPlan& pl, int p);
+// fills f and returns true if the box runs the phases of wb_plane.cuh
+bool rt_fast_setup(int nx, int ny, RtFast* f);
 // shared memory of the runtime plane kernels for the given geometry and element size
 size_t rt_plane_smem(const RtGeo& g, int elem_bytes, int* rows_per_chunk);
 
@@ -87,7 +101,7 @@ void rt_plane_inv_box(const FftArgs& f, const double2* sticks, int nitems, doubl
 void rt_plane_rhs(const FftArgs& f, const double2* evcr, const double2* dvbox, int npv, int mb, double2* sticks);
 void rt_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evcr, const double* occ, int nocc,
                    int mb, double2* acc, double scale, double2* osticks);
-void rt_setup(const RtGeo& g);
+void rt_setup();
 
 // SMs of the current device
 int sm_count();

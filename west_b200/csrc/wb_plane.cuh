@@ -57,6 +57,26 @@ struct CPlane {
   WB_DEV static constexpr bool dead(int n1) { return PR && !(n1 < A / 4 || n1 >= A - A / 4); }
 };
 
+// Geometry of any other box: edges and splits taken at run time, no pruning
+// beyond the active columns.
+struct RPlane {
+  static constexpr bool PR = false;
+  int nx_, ny_, ax_, bx_, ay_, by_, ncols_, nlow_;
+  unsigned mcols_, mrows_;  // ceil(2^32 / d): i / d = mulhi(i, m) for i d < 2^32
+  WB_DEV int ncols() const { return ncols_; }
+  WB_DEV int nlow() const { return nlow_; }
+  WB_DEV int nx() const { return nx_; }
+  WB_DEV int ny() const { return ny_; }
+  WB_DEV int ax() const { return ax_; }
+  WB_DEV int bx() const { return bx_; }
+  WB_DEV int ay() const { return ay_; }
+  WB_DEV int by() const { return by_; }
+  WB_DEV int rs() const { return nx_ | 1; }
+  WB_DEV int div_cols(int i) const { return (int)__umulhi((unsigned)i, mcols_); }
+  WB_DEV int div_rows(int i) const { return (int)__umulhi((unsigned)i, mrows_); }
+  WB_DEV static constexpr bool dead(int) { return false; }
+};
+
 // Step factors W_N^(k1 n2) at k1 B + n2 as a kernel parameter.
 template <int N, class C>
 struct TwParam {
@@ -204,6 +224,41 @@ WB_DEV void plane_row_box(const C* pl, C* __restrict__ o, const G& g, int nt) {
     row_to_real<B>(pl + y * rs + B * k1, v);
 #pragma unroll
     for (int i = 0; i < B; ++i) o[(k1 + A * i) * ny + y] = v[i];
+  }
+}
+// rows: inverse b) and the density sum += occ psi(r) dpsi(r) of a band pair, in
+// global memory, one element per thread throughout (first: the sum starts here)
+template <int B, class G, class C>
+WB_DEV void plane_row_density(const C* pl, const C* __restrict__ ps, real_t<C>* __restrict__ sum, real_t<C> o1,
+                              real_t<C> o2, bool first, const G& g, int nt) {
+  const int A = g.ax(), ny = g.ny(), rs = g.rs();
+  for (int it = threadIdx.x; it < ny * A; it += nt) {
+    const int k1 = g.div_rows(it), y = it - k1 * ny;
+    C v[B];
+    row_to_real<B>(pl + y * rs + B * k1, v);
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      const int e = (k1 + A * i) * ny + y;
+      const C s = ps[e];
+      const real_t<C> d = fma(o1 * s.x, v[i].x, o2 * s.y * v[i].y);
+      sum[e] = first ? d : sum[e] + d;
+    }
+  }
+}
+// rows: two real arrays (a + i b) scale -> forward B-point step
+template <int B, class G, class TW, class C>
+WB_DEV void plane_row_pair(C* pl, const TW& tx, const real_t<C>* a, const real_t<C>* b, real_t<C> scale, const G& g,
+                           int nt) {
+  const int A = g.ax(), ny = g.ny(), rs = g.rs();
+  for (int it = threadIdx.x; it < ny * A; it += nt) {
+    const int k1 = g.div_rows(it), y = it - k1 * ny;
+    C v[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      const int e = (k1 + A * i) * ny + y;
+      v[i] = mkc<C>(a[e] * scale, b ? b[e] * scale : real_t<C>(0));
+    }
+    row_from_real<B>(pl + y * rs + B * k1, v, tx, k1);
   }
 }
 // rows: psi(r) dv(r) scale (dv: the real or the imaginary part of d) -> forward B-point step
