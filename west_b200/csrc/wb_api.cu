@@ -136,7 +136,31 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
     if (upload(colx.data(), colx.size(), c->rt_colx) || upload(spos.data(), spos.size(), c->stpos))
       return fail(WB_ERR_NOMEM, "device allocation failed");
   }
+  // z runs of the compiled z passes: every pair's coefficients on side 0, z
+  // consecutive (pair 0: from z = 0), or a table of [pair][z]
+  std::vector<int> zlo(nsp, 0), zmap;
+  bool runs = true;
+  for (int p = 0; p < nsp; ++p) {
+    zlo[p] = spg[p] < spg[p + 1] ? gqz[spg[p]].y : 0;
+    for (int g = spg[p]; g < spg[p + 1]; ++g) runs = runs && (gqz[g].x & 1) == 0 && gqz[g].y == zlo[p] + g - spg[p];
+  }
+  runs = runs && zlo[0] == 0;
+  if (!runs && !rt) {
+    zmap.assign((size_t)nsp * N, -1);
+    for (int g = 0; g < npw; ++g) {
+      const int q = gqz[g].x / 2, side = gqz[g].x & 1, z = gqz[g].y;
+      int* m = zmap.data() + (size_t)q * N;
+      if (q == 0) {
+        m[(z + N) % N] = 2 * g + (z == 0);
+        if (z) m[(N - z) % N] = 2 * g + 1;
+      } else {
+        m[((side ? -z : z) + N) % N] = 2 * g + side;
+      }
+    }
+  }
   // device copies
+  if (upload(zlo.data(), zlo.size(), c->zlo) || (!zmap.empty() && upload(zmap.data(), zmap.size(), c->zmap)))
+    return fail(WB_ERR_NOMEM, "device allocation of stick tables failed");
   if (c->gqz.ensure(sizeof(int2) * npw) || c->spg.ensure(sizeof(int) * (nsp + 1)) ||
       c->cmap.ensure(sizeof(int) * cmap.size()) || c->perm.ensure(sizeof(int) * npw))
     return fail(WB_ERR_NOMEM, "device allocation of stick tables failed");
@@ -150,6 +174,11 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
   c->st.g_qz = c->gqz.as<int2>();
   c->st.hs = hs;
   c->st.cmap = c->cmap.as<int>();
+  c->st.gmax = 0;
+  for (int p = 0; p < nsp; p += kZGroup)
+    c->st.gmax = std::max(c->st.gmax, spg[std::min(p + kZGroup, nsp)] - spg[p]);
+  c->st.zlo = c->zlo.as<int>();
+  c->st.zmap = zmap.empty() ? nullptr : c->zmap.as<int>();
   c->st.prune = prune;
   if (rt) {
     if (ncols < 2) c->geo.fast = nullptr;  // RPlane divides by multiplication, which has no 1
@@ -1229,7 +1258,7 @@ int wb_ctx_destroy(wb_ctx* c) {
   if (!c) return WB_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  DBuf* bufs[] = {&c->perm, &c->gqz, &c->spg, &c->stpos, &c->cmap, &c->tw, &c->g2kin, &c->sqvc, &c->vs, &c->evc, &c->W,
+  DBuf* bufs[] = {&c->perm, &c->gqz, &c->spg, &c->stpos, &c->cmap, &c->zlo, &c->zmap, &c->tw, &c->g2kin, &c->sqvc, &c->vs, &c->evc, &c->W,
                   &c->D, &c->eprec, &c->et, &c->occ, &c->evcr, &c->iprec, &c->dvg_in, &c->dng_out, &c->aux, &c->dvbox, &c->B,
                   &c->X, &c->G, &c->T, &c->sticks, &c->sticks2, &c->acc, &c->part, &c->C, &c->rho, &c->conv,
                   &c->act, &c->items, &c->nact, &c->ecol, &c->epcol, &c->unconv, &c->items_pp, &c->items_pk,

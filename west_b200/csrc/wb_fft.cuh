@@ -226,7 +226,6 @@ struct LinePad {
 // k1 + N1*k2 is live iff k2 is in the outer quarters (needs N2 % 4 == 0).
 // Dead inputs are compile-time zeros and dead outputs are never stored, so the
 // compiler removes their arithmetic.
-enum : int { PRUNE_NONE = 0, PRUNE_IN = 1, PRUNE_OUT = 2 };
 template <int N>
 struct Prune {
   static constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2;
@@ -235,53 +234,5 @@ struct Prune {
   WB_DEV static constexpr bool in_live(int n1) { return n1 < N1 / 4 || n1 >= N1 - N1 / 4; }
   WB_DEV static constexpr bool out_live(int k2) { return k2 < N2 / 4 || k2 >= N2 - N2 / 4; }
 };
-
-// Batched line FFTs in shared memory (the z passes).  Line l starts at
-// data + l * stride, its elements in the LinePad layout.  Step 1 gives
-// consecutive threads consecutive n2 of a line, step 2 consecutive k1.  Both
-// must be called by all NT threads of the block.
-template <int N, int DIR, int NT, int PRUNE = PRUNE_NONE, class C>
-WB_DEV void fft_lines(C* data, int stride, int nlines, const C* twN) {
-  using LP = LinePad<N>;
-  using PR = Prune<N>;
-  constexpr bool PIN = (PRUNE == PRUNE_IN) && PR::IN_OK;
-  constexpr bool POUT = (PRUNE == PRUNE_OUT) && PR::OUT_OK;
-  constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2;
-  const int tid = threadIdx.x;
-  for (int it = tid; it < nlines * N2; it += NT) {
-    const int line = it / N2, n2 = it % N2;
-    C* p = data + line * stride;
-    C v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1)
-      v[n1] = (PIN && !PR::in_live(n1)) ? mkc<C>(0, 0) : p[LP::off_blk(n1, n2)];
-    rdft<N1, DIR>(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) v[k1] = ctw<DIR>(v[k1], twN[k1 * N2 + n2]);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) p[LP::off_blk(k1, n2)] = v[k1];
-  }
-  __syncthreads();
-  constexpr int LPC = NT / N1;
-  const int nchunks = (nlines + LPC - 1) / LPC;
-  for (int c = 0; c < nchunks; ++c) {
-    const int line = c * LPC + tid / N1, k1 = tid % N1;
-    const bool act = (tid < LPC * N1) && (line < nlines);
-    C v[N2];
-    C* p = data + (act ? line * stride : 0);
-    if (act) {
-#pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[LP::off_blk(k1, n2)];
-      rdft<N2, DIR>(v);
-    }
-    __syncthreads();
-    if (act) {
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2)
-        if (!POUT || PR::out_live(k2)) p[LP::off(k1 + N1 * k2)] = v[k2];
-    }
-  }
-  __syncthreads();
-}
 
 }  // namespace wb

@@ -30,193 +30,216 @@
 
 namespace wb {
 
-// z passes: 8 stick pairs per CTA of 128 threads (measured against 16/256 and
-// 4/64 at 64^3: more, smaller CTAs overlap one CTA's loads with another's
-// transform and stores; zfwd 0.30 instead of 0.34 us per FP64 item)
-constexpr int ZSG = 8;
-constexpr int ZNT = 128;
-
-// step-1 factor table of a line (wb_fft.cuh) into shared memory
-template <int N, class C>
-WB_DEV void load_tw(C* tw, const C* twg) {
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twg[i];
-}
-
 // ---------------------------------------------------------------------------
-// z pass, inverse: sphere coefficients of a pair of columns -> sticks
+// z passes
 // ---------------------------------------------------------------------------
-// One unit = stick pairs [ZSG qg, ZSG qg + ZSG) of band-pair item `item`.
-// Shared memory of every unit: the twiddles (N), then the work area.
-// Line side * ZSG + i of the work area is that stick of pair q0 + i.  A unit
-// takes its pointers from the dynamic shared array itself so that a unit body
-// compiled as a separate function still addresses shared memory directly.
+// One unit = stick pairs [ZSG qg, ZSG qg + ZSG) of band-pair item `item`; line
+// side * ZSG + i of its work area is that stick of pair q0 + i.  The four-step
+// transforms keep everything but the exchange between the two steps in
+// registers: the inverse's first step takes the sphere's coefficients straight
+// from global memory (consecutive threads along a stick, whose coefficients are
+// one run) and its second stores the sticks (consecutive threads over sticks);
+// the forward's first step reads the sticks the same way, and in its second a
+// thread owns z = k1 + A k2 of a stick and -z of its mirror, which is what the
+// Gamma unpack of those G needs.
+// Two steps of shared memory and one barrier per transform, where a zeroed and
+// scattered work area, in-place steps and a separate unpack took five and three.
+// Bound by DRAM latency and bandwidth: per item on one B200, inverse and forward,
+// 64^3 FP32 0.143 and 0.170 us (0.188 and 0.199 before; 0.08 and 0.10 at 6.65
+// TB/s), FP64 0.237 and 0.271 (0.238 and 0.302; 0.16 and 0.20); 108^3 FP64 1.42
+// and 1.61 (1.53 and 1.76), FP32 0.70 and 0.84 (0.82 and 0.90).
+constexpr int ZSG = kZGroup;
+
 template <class C>
 WB_DEV C* smem_tw() {
   extern __shared__ __align__(16) unsigned char smraw[];
   return reinterpret_cast<C*>(smraw);
 }
-
-// Twiddles of one thread, held in registers so that their global loads are
-// issued with the unit's other loads and stored to shared memory after the zero
-// fill.
+// step factor table of a line (wb_fft.cuh) into shared memory
 template <int N, class C>
-struct TwRegs {
-  static constexpr int PER = (N + ZNT - 1) / ZNT;
-  C v[PER];
-  WB_DEV void load(const C* __restrict__ twg) {
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int i = threadIdx.x + ZNT * k;
-      if (i < N) v[k] = twg[i];
-    }
-  }
-  WB_DEV void store(C* tw) const {
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int i = threadIdx.x + ZNT * k;
-      if (i < N) tw[i] = v[k];
-    }
-  }
-};
+WB_DEV void load_tw(C* tw, const C* twg) {
+  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twg[i];
+}
+// threads: the inverse's first step has ZSG B items; the forward's has 2 ZSG B
+template <int N>
+constexpr int z_threads() {
+  constexpr int m = FftSplit<N>::N1 > FftSplit<N>::N2 ? FftSplit<N>::N1 : FftSplit<N>::N2;
+  return (ZSG * m + 31) / 32 * 32;
+}
+// items, except where those threads would each hold two FP64 DFTs of 10 or more
+// points in the second (80^3: 160 threads 0.91 us per item, 96 threads 0.78)
+template <int N, class C>
+constexpr int zf_threads() {
+  return sizeof(C) == 16 && FftSplit<N>::N2 >= 10 ? z_threads<N>() : (2 * ZSG * FftSplit<N>::N2 + 31) / 32 * 32;
+}
 
-// G coefficients prefetched per thread before the zero fill (the rest of a
-// stick group's G vectors, if any, are read in a second loop).
-constexpr int kZPre = 2;
-
-static_assert((ZSG & (ZSG - 1)) == 0, "z_line's mirror flips one bit");
-// line of pair-and-side 2 i + side of a stick group
-WB_DEV int z_line(int l) { return (l & 1) * ZSG + (l >> 1); }
-
-template <int N, bool PR, class C>
-__global__ void __launch_bounds__(ZNT) k_zinv(const C* __restrict__ src, long ld,
-                                              const int2* __restrict__ items, StickTab st,
-                                              C* __restrict__ out,
-                                              const C* __restrict__ twg, const int* dn) {
-  if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;  // beyond the device item count
-  constexpr int LS = LinePad<N>::LEN | 1;  // odd line stride: conflict-free transposes
-  using LP = LinePad<N>;
-  C* tw = smem_tw<C>();
-  C* zb = smem_tw<C>() + N;
-  const int qg = blockIdx.x, item = blockIdx.y;
-  const int q0 = qg * ZSG;
-  const int nq = min(ZSG, st.nsp - q0);
-  const int2 it = items[item];
-  const C* a = src + (long)it.x * ld;
-  const C* b = src + (long)(it.y >= 0 ? it.y : it.x) * ld;
-  const bool two = it.y >= 0;
-  const int g0 = st.sp_gstart[q0], g1 = st.sp_gstart[q0 + nq];
-  TwRegs<N, C> twr;
-  twr.load(twg);
-  C pa[kZPre], pb[kZPre];
-  int2 pq[kZPre];
-#pragma unroll
-  for (int k = 0; k < kZPre; ++k) {
-    const int g = g0 + threadIdx.x + k * ZNT;
-    if (g < g1) {
-      pq[k] = st.g_qz[g];
-      pa[k] = a[g];
-      pb[k] = two ? b[g] : mkc<C>(0, 0);
-    }
-  }
-  // zero what step 1 reads: with pruning only the live inputs (the sphere's z
-  // lie in the outer quarters), otherwise the whole lines
-  if constexpr (PR && Prune<N>::IN_OK) {
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, NLIVE = N1 / 2;
-    for (int e = threadIdx.x; e < 2 * ZSG * NLIVE * N2; e += ZNT) {
-      const int l = e / (NLIVE * N2), r = e % (NLIVE * N2);
-      const int h = r / N2, n2 = r % N2;
-      const int n1 = h < NLIVE / 2 ? h : N1 - NLIVE + h;
-      zb[l * LS + LP::off_blk(n1, n2)] = mkc<C>(0, 0);
-    }
+// The G vector behind element zi of the side-0 stick of pair q: g, or -1; flip:
+// the sphere stores -G instead (for pair 0, its own mirror, also at G = 0, where
+// the -G store wins as in the reference loop).  Without MAP each pair's
+// coefficients are one ascending run of side 0, as in every sphere cut by planes;
+// MAP reads a table instead (any half of the sphere).
+template <int N, bool MAP>
+WB_DEV int z_lookup(const StickTab& st, int q, int zi, bool* flip) {
+  if constexpr (MAP) {
+    const int e = __ldg(st.zmap + (long)q * N + zi);
+    *flip = e & 1;
+    return e >> 1;  // -1 stays -1
   } else {
-    for (int i = threadIdx.x; i < 2 * ZSG * LS; i += ZNT) zb[i] = mkc<C>(0, 0);
-  }
-  twr.store(tw);
-  __syncthreads();
-  auto put = [&](int2 qz, C a1, C a2) {
-    // pos = a1 + i a2 ; neg = conj(a1 - i a2)
-    const C pos = mkc<C>(a1.x - a2.y, a1.y + a2.x);
-    const C neg = mkc<C>(a1.x + a2.y, a2.x - a1.y);
-    const int z = qz.y;
-    if (qz.x < 2) {  // the (0,0) stick is its own mirror
-      if (z != 0) { zb[LP::off((z + N) % N)] = pos; zb[LP::off((N - z) % N)] = neg; }
-      else zb[0] = neg;  // G = 0: the -G store wins, as in the reference loop
-    } else {
-      const int l = z_line(qz.x - 2 * q0);  // line of the stick holding G; its mirror is l ^ ZSG
-      zb[l * LS + LP::off((z + N) % N)] = pos;
-      zb[(l ^ ZSG) * LS + LP::off((N - z) % N)] = neg;
-    }
-  };
-#pragma unroll
-  for (int k = 0; k < kZPre; ++k)
-    if (g0 + (int)threadIdx.x + k * ZNT < g1) put(pq[k], pa[k], pb[k]);
-  for (int g = g0 + threadIdx.x + kZPre * ZNT; g < g1; g += ZNT)
-    put(st.g_qz[g], a[g], two ? b[g] : mkc<C>(0, 0));
-  __syncthreads();
-  fft_lines<N, +1, ZNT, PR ? PRUNE_IN : PRUNE_NONE>(zb, LS, 2 * ZSG, tw);
-  C* o = out + (long)item * N * st.nst + q0;
-  for (int e = threadIdx.x; e < 2 * ZSG * N; e += ZNT) {
-    const int l = e % (2 * ZSG), z = e / (2 * ZSG);
-    if (l % ZSG < nq) o[(long)z * st.nst + (l / ZSG) * st.hs + l % ZSG] = zb[l * LS + LinePad<N>::off(z)];
+    int z = zi < (N + 1) / 2 ? zi : zi - N;
+    const int g0 = __ldg(st.sp_gstart + q), n = __ldg(st.sp_gstart + q + 1) - g0;
+    *flip = q == 0 && z <= 0;
+    if (q == 0) z = z < 0 ? -z : z;
+    const int i = z - __ldg(st.zlo + q);
+    return i >= 0 && i < n ? g0 + i : -1;
   }
 }
 
-// ---------------------------------------------------------------------------
-// z pass, forward: sticks -> sphere with the Gamma unpack, then an epilogue
-// ---------------------------------------------------------------------------
-// An epilogue reads its per-G inputs through Epi::pre (prefetching them
-// before the transform was measured slower: the extra registers cost more
-// occupancy than the hidden latency gained).
-template <int N, bool PR, class C, class Epi>
-__global__ void __launch_bounds__(ZNT) k_zfwd(const C* __restrict__ sticks,
-                                              const int2* __restrict__ items, StickTab st,
-                                              const C* __restrict__ twg, Epi epi, const int* dn) {
+template <int N, bool PR, class C, bool MAP>
+__global__ void __launch_bounds__(z_threads<N>()) k_zinv(const C* __restrict__ src, long ld,
+                                                         const int2* __restrict__ items, StickTab st,
+                                                         C* __restrict__ out, const C* __restrict__ twg,
+                                                         const int* dn) {
+  if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;  // beyond the device item count
+  constexpr int A = FftSplit<N>::N1, B = FftSplit<N>::N2, NT = z_threads<N>();
+  constexpr int LS = LinePad<N>::LEN | 1;  // odd: the second step's lanes over lines hit distinct banks
+  using LP = LinePad<N>;
+  using P = Prune<N>;
+  constexpr bool PIN = PR && P::IN_OK;
+  C* tw = smem_tw<C>();
+  C* zb = tw + N;
+  const int q0 = blockIdx.x * ZSG, item = blockIdx.y;
+  const int nq = min(ZSG, st.nsp - q0);
+  const int2 it2 = items[item];
+  const C* a = src + (long)it2.x * ld;
+  const bool two = it2.y >= 0;
+  const C* b = src + (long)(two ? it2.y : it2.x) * ld;
+  load_tw<N>(tw, twg);
+  __syncthreads();
+  for (int it = threadIdx.x; it < nq * B; it += NT) {
+    const int i = it / B, n2 = it % B, q = q0 + i;
+    C v0[A], v1[A];  // element B n1 + n2 of side 0, and of side 1 at its negative
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) {
+      v0[n1] = v1[n1] = mkc<C>(0, 0);
+      if (!PIN || P::in_live(n1)) {
+        bool flip;
+        const int g = z_lookup<N, MAP>(st, q, B * n1 + n2, &flip);
+        if (g >= 0) {
+          const C a1 = a[g], a2 = two ? b[g] : mkc<C>(0, 0);
+          const C pos = mkc<C>(a1.x - a2.y, a1.y + a2.x);  // a1 + i a2
+          const C neg = mkc<C>(a1.x + a2.y, a2.x - a1.y);  // conj(a1 - i a2)
+          v0[n1] = flip ? neg : pos;
+          v1[n1] = flip ? pos : neg;
+        }
+      }
+    }
+    C w[A];
+#pragma unroll
+    for (int j = 0; j < A; ++j) w[j] = n2 == 0 ? v1[(A - j) % A] : v1[A - 1 - j];
+    C* p = zb + i * LS;
+    rdft<A, +1>(v0);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) p[LP::off_blk(k1, n2)] = k1 ? ctw<+1>(v0[k1], tw[k1 * B + n2]) : v0[0];
+    const int m2 = n2 == 0 ? 0 : B - n2;
+    p += ZSG * LS;
+    rdft<A, +1>(w);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) p[LP::off_blk(k1, m2)] = k1 ? ctw<+1>(w[k1], tw[k1 * B + m2]) : w[0];
+  }
+  __syncthreads();
+  C* o = out + (long)item * N * st.nst + q0;
+  for (int it = threadIdx.x; it < 2 * ZSG * A; it += NT) {
+    const int l = it % (2 * ZSG), k1 = it / (2 * ZSG);
+    if (l % ZSG >= nq) continue;
+    const C* p = zb + l * LS;
+    C v[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) v[n2] = p[LP::off_blk(k1, n2)];
+    rdft<B, +1>(v);
+    C* os = o + (l / ZSG) * st.hs + l % ZSG;
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) os[(long)(k1 + A * k2) * st.nst] = v[k2];
+  }
+}
+
+// sticks -> sphere with the Gamma unpack, then an epilogue per G.  The columns an
+// epilogue reads are copied to shared memory behind the first step (one run of G
+// for the whole stick group), so that it waits for none of them.
+template <int N, bool PR, class C, class Epi, bool MAP>
+__global__ void __launch_bounds__(zf_threads<N, C>()) k_zfwd(const C* __restrict__ sticks,
+                                                         const int2* __restrict__ items, StickTab st,
+                                                         const C* __restrict__ twg, Epi epi, const int* dn) {
   if (dn && (int)blockIdx.y >= dev_count<true>(dn, 0)) return;
+  constexpr int A = FftSplit<N>::N1, B = FftSplit<N>::N2, NT = zf_threads<N, C>();
   constexpr int LS = LinePad<N>::LEN | 1;
   using LP = LinePad<N>;
   using T = real_t<C>;
+  using P = Prune<N>;
+  constexpr bool POUT = PR && P::OUT_OK;
   C* tw = smem_tw<C>();
-  C* zb = smem_tw<C>() + N;
-  const int qg = blockIdx.x, item = blockIdx.y;
-  const int q0 = qg * ZSG;
+  C* zb = tw + N;
+  const int q0 = blockIdx.x * ZSG, item = blockIdx.y;
   const int nq = min(ZSG, st.nsp - q0);
   const C* s0 = sticks + (long)item * N * st.nst + q0;
-  // asynchronous copies: all of a CTA's reads are in flight at once, without
-  // registers (a loop of loads and stores left the kernel waiting for each)
-  for (int e = threadIdx.x; e < 2 * ZSG * N; e += ZNT) {
-    const int l = e % (2 * ZSG), z = e / (2 * ZSG);
-    if (l % ZSG < nq)
-      cp_async_elem(zb + l * LS + LinePad<N>::off(z), s0 + (long)z * st.nst + (l / ZSG) * st.hs + l % ZSG);
-  }
-  load_tw<N>(tw, twg);
-  const int2 it = items[item];
-  const int g0 = st.sp_gstart[q0], g1 = st.sp_gstart[q0 + nq];
-  cp_async_wait_all();
-  __syncthreads();
-  fft_lines<N, -1, ZNT, PR ? PRUNE_OUT : PRUNE_NONE>(zb, LS, 2 * ZSG, tw);
-  auto take = [&](int g, int2 qz, const typename Epi::Pre& pr) {
-    const int z = qz.y;
-    C ap, am;
-    if (qz.x < 2) {
-      ap = zb[LP::off((z + N) % N)];
-      am = zb[LP::off((N - z) % N)];
-    } else {
-      const int l = z_line(qz.x - 2 * q0);
-      ap = zb[l * LS + LP::off((z + N) % N)];
-      am = zb[(l ^ ZSG) * LS + LP::off((N - z) % N)];
+  const int2 it2 = items[item];
+  const int g0 = st.sp_gstart[q0], ng = st.sp_gstart[q0 + nq] - g0;
+  C* ps = zb + 2 * ZSG * LS;
+  if constexpr (Epi::STAGED)
+    for (int i = threadIdx.x; i < ng; i += NT) {
+      cp_async_elem(ps + i, epi.P + (long)it2.x * epi.ld + g0 + i);
+      if (it2.y >= 0) cp_async_elem(ps + ng + i, epi.P + (long)it2.y * epi.ld + g0 + i);
     }
-    const C fp = mkc<C>(T(0.5) * (ap.x + am.x), T(0.5) * (ap.y + am.y));
-    const C fm = mkc<C>(T(0.5) * (ap.x - am.x), T(0.5) * (ap.y - am.y));
-    epi(g, it, pr, mkc<C>(fp.x, fm.y), mkc<C>(fp.y, -fm.x));
-  };
-  for (int g = g0 + threadIdx.x; g < g1; g += ZNT) take(g, st.g_qz[g], epi.pre(g, it));
+  load_tw<N>(tw, twg);
+  __syncthreads();
+  for (int it = threadIdx.x; it < 2 * ZSG * B; it += NT) {
+    const int l = it % (2 * ZSG), n2 = it / (2 * ZSG);
+    if (l % ZSG >= nq) continue;
+    const C* is = s0 + (l / ZSG) * st.hs + l % ZSG;
+    C v[A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) v[n1] = is[(long)(B * n1 + n2) * st.nst];
+    rdft<A, -1>(v);
+    C* p = zb + l * LS;
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) p[LP::off_blk(k1, n2)] = k1 ? ctw<-1>(v[k1], tw[k1 * B + n2]) : v[0];
+  }
+  if constexpr (Epi::STAGED) cp_async_wait_all();
+  __syncthreads();
+  for (int it = threadIdx.x; it < nq * A; it += NT) {
+    const int i = it / A, k1 = it % A, q = q0 + i;
+    const int m1 = k1 == 0 ? 0 : A - k1;
+    const C* p0 = zb + i * LS;
+    const C* p1 = q == 0 ? p0 : p0 + ZSG * LS;  // the (0,0) stick is its own mirror
+    C v[B], u[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+      v[n2] = p0[LP::off_blk(k1, n2)];
+      u[n2] = p1[LP::off_blk(m1, n2)];
+    }
+    rdft<B, -1>(v);
+    rdft<B, -1>(u);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) {
+      if (POUT && !P::out_live(k2)) continue;
+      const int zi = k1 + A * k2;
+      bool flip;
+      const int g = z_lookup<N, MAP>(st, q, zi, &flip);
+      if (g < 0 || (q == 0 && flip && zi != 0)) continue;  // pair 0: each G once
+      const C s = k1 == 0 ? u[(B - k2) % B] : u[B - 1 - k2];
+      const C ap = flip ? s : v[k2], am = flip ? v[k2] : s;
+      const C fp = mkc<C>(T(0.5) * (ap.x + am.x), T(0.5) * (ap.y + am.y));
+      const C fm = mkc<C>(T(0.5) * (ap.x - am.x), T(0.5) * (ap.y - am.y));
+      epi(g, it2, epi.pre(g, it2, ps + (g - g0), ng), mkc<C>(fp.x, fm.y), mkc<C>(fp.y, -fm.x));
+    }
+  }
 }
 
 struct EpiStore {
   double2* dst;
   long ld;
+  static constexpr bool STAGED = false;
   struct Pre {};
-  WB_DEV Pre pre(int, int2) const { return {}; }
+  WB_DEV Pre pre(int, int2, const double2*, int) const { return {}; }
   WB_DEV void operator()(int g, int2 it, const Pre&, double2 b1, double2 b2) const {
     dst[(long)it.x * ld + g] = b1;
     if (it.y >= 0) dst[(long)it.y * ld + g] = b2;
@@ -237,10 +260,11 @@ struct EpiHpsiT {
     C p1, p2;
     T k;
   };
-  WB_DEV Pre pre(int g, int2 it) const {
+  static constexpr bool STAGED = true;
+  WB_DEV Pre pre(int g, int2 it, const C* ps, int ng) const {
     Pre r;
-    r.p1 = P[(long)it.x * ld + g];
-    r.p2 = it.y >= 0 ? P[(long)it.y * ld + g] : mkc<C>(0, 0);
+    r.p1 = ps[0];
+    r.p2 = it.y >= 0 ? ps[ng] : mkc<C>(0, 0);
     r.k = g2kin[g];
     return r;
   }
@@ -269,7 +293,8 @@ struct EpiDng {
     double s;
     int r;
   };
-  WB_DEV Pre pre(int g, int2) const { return {(g == 0) ? 0.0 : sqvc[g], perm[g]}; }
+  static constexpr bool STAGED = false;
+  WB_DEV Pre pre(int g, int2, const double2*, int) const { return {(g == 0) ? 0.0 : sqvc[g], perm[g]}; }
   WB_DEV void operator()(int g, int2 it, const Pre& pr, double2 b1, double2 b2) const {
     const double s = pr.s;
     const long r = pr.r;
@@ -563,25 +588,30 @@ struct FftN {
   static void smem(K* k, size_t bytes) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   }
+  template <bool PR, bool MAP>
+  static void setup_z() {
+    smem(k_zinv<N, PR, double2, MAP>, zsmem<N>());
+    smem(k_zfwd<N, PR, double2, EpiStore, MAP>, zsmem<N>());
+    smem(k_zfwd<N, PR, double2, EpiHpsi, MAP>, zsmem<N>() + 2 * sizeof(double2) * ZSG * N);
+    smem(k_zfwd<N, PR, double2, EpiDng, MAP>, zsmem<N>());
+    smem(k_zinv<N, PR, float2, MAP>, zsmem<N, float2>());
+    smem(k_zfwd<N, PR, float2, EpiHpsi32, MAP>, zsmem<N, float2>() + 2 * sizeof(float2) * ZSG * N);
+  }
   template <bool PR>
   static void setup_pr() {
-    smem(k_zinv<N, PR, double2>, zsmem<N>());
-    smem(k_zfwd<N, PR, double2, EpiStore>, zsmem<N>());
-    smem(k_zfwd<N, PR, double2, EpiHpsi>, zsmem<N>());
-    smem(k_zfwd<N, PR, double2, EpiDng>, zsmem<N>());
+    setup_z<PR, false>();
     smem(k_plane_vloc<N, PR, double2, false>, psmem<N, double2>());
     if constexpr (plane_blocks<N, double2>() == 1) smem(k_plane_vloc<N, PR, double2, true>, kMaxSmem);
     if constexpr (plane_blocks<N, float2>() == 1) smem(k_plane_vloc<N, PR, float2, true>, kMaxSmem);
     smem(k_plane_inv_box<N, PR>, psmem<N, double2>());
     smem(k_plane_rhs<N, PR>, psmem<N, double2>());
     smem(k_plane_drho<N, PR>, psmem<N, double2>());
-    smem(k_zinv<N, PR, float2>, zsmem<N, float2>());
-    smem(k_zfwd<N, PR, float2, EpiHpsi32>, zsmem<N, float2>());
     smem(k_plane_vloc<N, PR, float2, false>, psmem<N, float2>());
   }
   static void setup() {
     setup_pr<false>();
     setup_pr<true>();
+    setup_z<false, true>();
   }
   static dim3 zgrid(const StickTab& st, int nitems) { return dim3((st.nsp + ZSG - 1) / ZSG, nitems); }
   // Local-potential transforms of the PCG operator, FP64 (C = double2) or the
@@ -592,10 +622,9 @@ struct FftN {
   static void zinv_t(const F& f, const C* src, long ld, const int2* items, int nitems, C* sticks) {
     if (nitems <= 0) return;
     constexpr size_t zs = zsmem<N, C>();
-    if (f.st.prune)
-      k_zinv<N, true, C><<<zgrid(f.st, nitems), ZNT, zs, f.stream>>>(src, ld, items, f.st, sticks, f.tw, f.dcount);
-    else
-      k_zinv<N, false, C><<<zgrid(f.st, nitems), ZNT, zs, f.stream>>>(src, ld, items, f.st, sticks, f.tw, f.dcount);
+    // a half sphere without runs takes the table form, unpruned
+    auto k = f.st.zmap ? k_zinv<N, false, C, true> : f.st.prune ? k_zinv<N, true, C, false> : k_zinv<N, false, C, false>;
+    k<<<zgrid(f.st, nitems), z_threads<N>(), zs, f.stream>>>(src, ld, items, f.st, sticks, f.tw, f.dcount);
   }
   template <class C, class F>
   static void vloc_t(const F& f, C* sticks, int nitems, const real_t<C>* vs) {
@@ -618,10 +647,10 @@ struct FftN {
   static void zfwd_t(const F& f, const C* sticks, const int2* items, int nitems, Epi epi) {
     if (nitems <= 0) return;
     constexpr size_t zs = zsmem<N, C>();
-    if (f.st.prune)
-      k_zfwd<N, true, C, Epi><<<zgrid(f.st, nitems), ZNT, zs, f.stream>>>(sticks, items, f.st, f.tw, epi, f.dcount);
-    else
-      k_zfwd<N, false, C, Epi><<<zgrid(f.st, nitems), ZNT, zs, f.stream>>>(sticks, items, f.st, f.tw, epi, f.dcount);
+    auto k = f.st.zmap ? k_zfwd<N, false, C, Epi, true>
+                       : f.st.prune ? k_zfwd<N, true, C, Epi, false> : k_zfwd<N, false, C, Epi, false>;
+    const size_t staged = Epi::STAGED ? 2 * sizeof(C) * f.st.gmax : 0;
+    k<<<zgrid(f.st, nitems), zf_threads<N, C>(), zs + staged, f.stream>>>(sticks, items, f.st, f.tw, epi, f.dcount);
   }
   static void zinv32(const FftArgs32& f, const float2* src, long ld, const int2* items, int nitems, float2* sticks) {
     zinv_t<float2>(f, src, ld, items, nitems, sticks);

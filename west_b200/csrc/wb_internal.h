@@ -7,12 +7,16 @@
 namespace wb {
 
 // Stick decomposition of the Gamma half sphere (built on the host from nl).
+constexpr int kZGroup = 8;  // stick pairs per CTA of the z passes
 struct StickTab {
   int nsp;               // stick pairs; pair 0 is the (0,0) stick
   int nst;               // sticks in the buffer = 2 * hs
   int hs;                // stick side * hs + q is side 0 or 1 of pair q (hs >= nsp)
   const int* sp_gstart;  // [nsp + 1] first internal G index of each pair
   const int2* g_qz;      // [npw] (2 * pair + side, signed z) of each internal G
+  int gmax;              // most G vectors of kZGroup consecutive pairs from a multiple of it
+  const int* zlo;        // [nsp] lowest z of each pair (its coefficients are a run of side 0)
+  const int* zmap;       // null, or where pairs have no such runs: [pair][z] 2 g + flip, -1 = none (z_lookup)
   const int* cmap;       // [y][active column] stick at (x, y), -1 = none
   int xhi;               // active plane columns: x in [0, xhi] and [N - (ncols - xhi - 1), N)
   int ncols;
