@@ -5,6 +5,8 @@ buckets of the captured loop, the step kernel's clusters of 1 to 8 CTAs (few
 systems of many plane waves), and boxes that run the plane phases with radices
 taken at run time.  Converged solves (tr2 far below the production threshold) in
 FP64 against the oracle at the tolerance of the other parity tests (1e-10)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -48,6 +50,23 @@ def test_projector_counts(natoms, nbnd):
                                 dion=0.2, seed=3), "cuda")
     assert s.nkb + s.nbnd_occ in (64, 65, 112, 113, 208)
     _check(s, 17)
+
+
+@pytest.mark.parametrize("total", [5634, 6144])
+def test_reduction_of_many_projectors(tiny, total):
+    """Projectors and bands whose sums take all of the 48 KB that the reduction has for
+    them: zero projectors before tiny's own leave its response as it is."""
+    s = tiny
+    nkb = total - s.nbnd_occ
+    vkb = np.zeros((s.npw, nkb), dtype=np.complex128, order="F")
+    vkb[:, nkb - s.nkb:] = s.vkb
+    deeq = np.zeros((nkb, nkb), order="F")
+    deeq[nkb - s.nkb:, nkb - s.nkb:] = s.deeq
+    dvg = perturbations(s, 2, seed=1)
+    ref, _ = O.apply_operator(s, dvg, 1e-20, maxiter=400)
+    got, ierr = _solve(dataclasses.replace(s, vkb=vkb, deeq=deeq), dvg)
+    assert (ierr == 0).all()
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-10
 
 
 @pytest.mark.parametrize("L,ecut,nr", [(13.0, 12.0, 32), (15.0, 20.0, 48), (17.0, 25.0, 60)])   # clusters of 2, 4, 8

@@ -429,6 +429,9 @@ void la_setup() {
                        TnTile<112, 64, 1, 4, 1, 16, 3>::SMEM);
   cudaFuncSetAttribute(k_gemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(double) * NN_STAGE * NN_ST);
+  // S of all projectors beside the kernel's static scratch, which together pass the
+  // 48 KB that a launch has without this: up to 6,144 projectors
+  cudaFuncSetAttribute(k_gamma_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
 }
 
 // ---------------------------------------------------------------------------
