@@ -149,3 +149,26 @@ def test_noalloc_rejects_the_mixed_form():
                                               None)
     assert rc == L.WB_ERR_UNSUPPORTED
     assert "FP64" in lib.wb_last_error().decode()
+
+
+@pytest.mark.parametrize("L,nr,first,last", [(10.0, 24, 75, 76), ((10.0, 10.0, 10.5), (24, 24, 25), 71, 74)])
+def test_noalloc_largest_calls(L, nr, first, last):
+    """The last perturbation counts that fit the scratch, which they do without the
+    padding sticks only, on a compiled and a run-time box; one more is refused."""
+    import torch
+    from west_b200 import lib as L_
+    from west_b200.system import SystemSpec
+    from west_b200.wstat import ResponseOperator
+
+    s = build_system(SystemSpec(L=L, ecutwfc=8.0, nr=nr, natoms=3, nbnd_occ=7, proj="sp", seed=12))
+    op = ResponseOperator(s, verbose=False, n_dfpt_maxiter=400)
+    dv = torch.from_numpy(np.ascontiguousarray(perturbations(s, last + 1, seed=3).T)).cuda()
+    for m in (first, last):
+        ref, eref = _device(op, m, dv, 1e-20)
+        got, ierr = _noalloc(op, m, dv[:m].contiguous(), s.npw, 1e-20)
+        assert (ierr == eref).all(), m
+        assert _rel(got, ref) < TOL_FP64, m
+    out = torch.zeros_like(dv)
+    rc = L_.load().wb_apply_operator_device_noalloc(op._ctx, last + 1, dv.data_ptr(), s.npw, out.data_ptr(), s.npw,
+                                                    1e-20, 1, None)
+    assert rc == L_.WB_ERR_ARG

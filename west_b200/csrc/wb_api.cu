@@ -117,17 +117,20 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
   c->st.xhi = prune ? N / 4 - 1 : xmax;
   c->st.ncols = prune ? N / 2 : 2 * xmax + 1;
   const int ncols = c->st.ncols, nlow = c->st.xhi + 1;
-  std::vector<int> cmap((size_t)n2 * ncols, -1), spos(nst, -1);
-  auto place = [&](int stick, int x, int y) {
+  // [0] with side 1 at hs, [1] with it at nsp (the tables of c->st and c->st_tight)
+  const size_t nmap = (size_t)n2 * ncols;
+  std::vector<int> cmap(2 * nmap, -1), spos(2 * nst, -1);
+  auto place = [&](int tight, int stick, int x, int y) {
     const int xb = (x + n1) % n1, yb = (y + n2) % n2;
     const int col = xb < nlow ? xb : xb - (n1 - ncols);
-    cmap[(size_t)yb * ncols + col] = stick;
-    if (rt) spos[stick] = (x + xmax) * (n2 | 1) + yb;
+    cmap[tight * nmap + (size_t)yb * ncols + col] = stick;
+    if (rt) spos[tight * nst + stick] = (x + xmax) * (n2 | 1) + yb;
   };
-  for (int p = 0; p < nsp; ++p) {
-    place(p, pair_xy[p].first, pair_xy[p].second);
-    if (p > 0) place(hs + p, -pair_xy[p].first, -pair_xy[p].second);
-  }
+  for (int tight = 0; tight < 2; ++tight)
+    for (int p = 0; p < nsp; ++p) {
+      place(tight, p, pair_xy[p].first, pair_xy[p].second);
+      if (p > 0) place(tight, (tight ? nsp : hs) + p, -pair_xy[p].first, -pair_xy[p].second);
+    }
   if (rt) {
     std::vector<int> colx(ncols);
     for (int cidx = 0; cidx < ncols; ++cidx) colx[cidx] = (cidx - xmax + n1) % n1;
@@ -185,6 +188,10 @@ int build_tables(wb_ctx* c, const wb_system* s, std::vector<int>& perm) {
     c->geo.colx = c->rt_colx.as<int>();
     c->geo.spos = c->stpos.as<int>();
   }
+  c->st_tight = c->st;
+  c->st_tight.hs = nsp;
+  c->st_tight.nst = 2 * nsp;
+  c->st_tight.cmap += nmap;
   return WB_OK;
 }
 
@@ -1205,6 +1212,8 @@ int wb_ctx_create(wb_ctx** out, const wb_system* s, int device) {
     c->geo.twx = c->twx.as<double2>();
     c->geo.twy = c->twy.as<double2>();
     c->geo.twz = c->twz.as<double2>();
+    c->geo_tight = c->geo;
+    c->geo_tight.spos += c->st.nst;
     if (rt_plane_smem(c->geo, 16, nullptr) == 0)
       return bail(fail(WB_ERR_UNSUPPORTED, "the x-y plane of this box does not fit in shared memory"));
   }
@@ -1437,19 +1446,28 @@ struct Carve {
 constexpr int kNoallocCtas = 2;  // the built-in split target
 
 struct NoallocWs {
+  FftArgs fa;  // the context's, or with its sticks unpadded
   double2 *aux, *dvbox, *B, *X, *G, *T, *sticks, *sticks2, *acc;
   double *part, *C, *rho, *ecol, *epcol;
   unsigned char* conv;
   int *act, *nact, *unconv;
   int2 *items, *items_pp, *items_pk;
-  bool plan;   // the bra-kets split as the other entry points' do; else nsplit ways
+  bool plan;   // the bra-kets split as the other entry points' do, else nsplit ways
   int nsplit;
 };
 
-void noalloc_layout(const wb_ctx* c, int mb, bool plan, Carve& cv, NoallocWs& w) {
+// level 0: the bra-kets split as in the other entry points; 1: with fewer splits, 2:
+// and without the sticks that pad the two sides of a plane to multiples of eight
+void noalloc_layout(const wb_ctx* c, int mb, int level, Carve& cv, NoallocWs& w) {
+  const bool plan = level == 0;
   const size_t nsys = (size_t)mb * c->nocc;
   const size_t npw = c->npw;
-  const size_t stk1 = (size_t)c->nz * c->st.nst;
+  w.fa = c->fa;
+  if (level == 2) {
+    w.fa.st = c->st_tight;
+    if (c->rt) w.fa.rt = &c->geo_tight;
+  }
+  const size_t stk1 = (size_t)c->nz * w.fa.st.nst;
   const size_t mp = ((size_t)mb + 1) / 2;
   const size_t nitems = std::max<size_t>({(nsys + 1) / 2, (size_t)mb * c->npv, mp});
   w.plan = plan;
@@ -1504,9 +1522,9 @@ void noalloc_apply_A(wb_ctx* c, const NoallocWs& w, const double2* Xv, double2* 
     nkb = 0;
   } else {
     const int nit = (n + 1) / 2;
-    fft_zinv(c->fa, Xv, ld, items, nit, w.sticks);
-    fft_plane_vloc(c->fa, w.sticks, nit, c->vs.as<double>());
-    fft_zfwd_hpsi(c->fa, w.sticks, items, nit, Xv, Tv, ld, c->g2kin.as<double>(), w.ecol);
+    fft_zinv(w.fa, Xv, ld, items, nit, w.sticks);
+    fft_plane_vloc(w.fa, w.sticks, nit, c->vs.as<double>());
+    fft_zfwd_hpsi(w.fa, w.sticks, items, nit, Xv, Tv, ld, c->g2kin.as<double>(), w.ecol);
   }
   const int ns = w.plan ? gemm_tn_plan(M, n, K, kNoallocCtas) : w.nsplit;
   gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, ns, w.part, s);
@@ -1528,10 +1546,10 @@ int noalloc_run(wb_ctx* c, const NoallocWs& w, int mb, const double2* dvg, long 
   fill_columns(c->et.as<double>(), nocc, nsys, w.ecol, s);
   fill_columns(c->eprec.as<double>(), nocc, nsys, w.epcol, s);
   permute_scale(dvg, ld_in, c->perm.as<int>(), c->sqvc.as<double>(), npw, mb, w.aux, ld, s);
-  fft_zinv(c->fa, w.aux, ld, w.items_pp, mp, w.sticks);
-  fft_plane_inv_box(c->fa, w.sticks, mp, w.dvbox);
-  fft_plane_rhs(c->fa, c->evcr.as<double2>(), w.dvbox, npv, mb, w.sticks);
-  fft_zfwd_store(c->fa, w.sticks, w.items_pk, mb * npv, w.B, ld);
+  fft_zinv(w.fa, w.aux, ld, w.items_pp, mp, w.sticks);
+  fft_plane_inv_box(w.fa, w.sticks, mp, w.dvbox);
+  fft_plane_rhs(w.fa, c->evcr.as<double2>(), w.dvbox, npv, mb, w.sticks);
+  fft_zfwd_store(w.fa, w.sticks, w.items_pk, mb * npv, w.B, ld);
   const double* Wevc = c->W.as<double>() + (size_t)c->nkb * K;
   const int ns = w.plan ? gemm_tn_plan(nocc, nsys, K, kNoallocCtas) : w.nsplit;
   gemm_tn(Wevc, K, nocc, (const double*)w.B, 2 * ld, nullptr, nsys, K, ns, w.part, s);
@@ -1565,10 +1583,10 @@ int noalloc_run(wb_ctx* c, const NoallocWs& w, int mb, const double2* dvg, long 
     WB_CU(cudaMemsetAsync(w.unconv, 0, sizeof(int) * mb, s));
   }
   c->stats.cg_iterations = std::max(c->stats.cg_iterations, iters);
-  fft_zinv(c->fa, w.X, ld, w.items_pk, mb * npv, w.sticks);
+  fft_zinv(w.fa, w.X, ld, w.items_pk, mb * npv, w.sticks);
   const double scale = 2.0 * c->wk / c->omega / (double)c->nnr;
-  fft_plane_drho(c->fa, w.sticks, c->evcr.as<double2>(), c->occ.as<double>(), nocc, mb, w.acc, scale, w.sticks2);
-  fft_zfwd_dng(c->fa, w.sticks2, w.items_pp, mp, dng, ld_out, c->perm.as<int>(), c->sqvc.as<double>());
+  fft_plane_drho(w.fa, w.sticks, c->evcr.as<double2>(), c->occ.as<double>(), nocc, mb, w.acc, scale, w.sticks2);
+  fft_zfwd_dng(w.fa, w.sticks2, w.items_pp, mp, dng, ld_out, c->perm.as<int>(), c->sqvc.as<double>());
   if (unconv_host) WB_CU(cudaMemcpyAsync(unconv_host, w.unconv, sizeof(int) * mb, cudaMemcpyDeviceToHost, s));
   WB_CU(cudaStreamSynchronize(s));
   WB_CU(cudaGetLastError());
@@ -1596,17 +1614,16 @@ extern "C" int wb_apply_operator_device_noalloc(wb_ctx* c, int m, const double* 
     return fail(WB_ERR_ARG, "m = " + std::to_string(m) + " perturbations do not fit the allocation-free entry "
                 "point's scratch of " + std::to_string((size_t)WB_NOALLOC_SCRATCH_BYTES) +
                 " bytes (WB_NOALLOC_SCRATCH_BYTES): use fewer perturbations per call");
-  // the split plan of the other entry points where its partial sums fit too, so
-  // that up to 64 systems give their bits; a call that fits only without them runs
-  // with fewer splits
+  // the first level that fits: with the split plan of the other entry points, up to
+  // 64 systems give their bits; unpadded sticks keep the largest calls within the
+  // scratch (75 perturbations of 7 bands at 24^3: 32.9 MB of 33.6, padded 34.2)
   Carve probe{nullptr};
   NoallocWs w{};
-  bool plan = true;
-  noalloc_layout(c, std::max(m, 1), plan, probe, w);
-  if (probe.off > (size_t)WB_NOALLOC_SCRATCH_BYTES) {
-    plan = false;
+  int level = 0;
+  noalloc_layout(c, std::max(m, 1), level, probe, w);
+  while (probe.off > (size_t)WB_NOALLOC_SCRATCH_BYTES && level < 2) {
     probe = Carve{nullptr};
-    noalloc_layout(c, std::max(m, 1), plan, probe, w);
+    noalloc_layout(c, std::max(m, 1), ++level, probe, w);
   }
   if (probe.off > (size_t)WB_NOALLOC_SCRATCH_BYTES)
     return fail(WB_ERR_ARG, "this call needs " + std::to_string(probe.off) + " bytes of scratch; the allocation-free "
@@ -1620,7 +1637,7 @@ extern "C" int wb_apply_operator_device_noalloc(wb_ctx* c, int m, const double* 
   c->stats.m = m;
   if (m == 0) return WB_OK;
   Carve cv{base};
-  noalloc_layout(c, m, plan, cv, w);
+  noalloc_layout(c, m, level, cv, w);
   if (ld_dng > c->npw)
     WB_CU(cudaMemset2DAsync(reinterpret_cast<double2*>(dng) + c->npw, sizeof(double2) * ld_dng, 0,
                             sizeof(double2) * (ld_dng - c->npw), m, c->stream));

@@ -62,6 +62,8 @@ struct wb_ctx {
   DBuf rt_colx, twx, twy, twz, twx32, twy32, twz32;
   double omega = 0, wk = 0, alpha = 0;
   wb::StickTab st{};
+  wb::StickTab st_tight{};   // the same without padding sticks (hs = nsp), and the geometry for it:
+  wb::RtGeo geo_tight{};     //   allocation-free calls that fit their scratch only so
   wb::FftArgs fa{};
   // constant device data
   DBuf perm, gqz, spg, stpos, cmap, zlo, zmap, tw, g2kin, sqvc, vs, evc, W, D, eprec, et, occ, evcr, iprec;
