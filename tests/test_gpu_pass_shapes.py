@@ -1,10 +1,10 @@
 """Shapes at which the kernels of a PCG pass change: the bra-ket's 32 x 32, 64 x 64
 and 112 x 64 tiles (64 | 65 systems, 64 | 65 and 112 | 113 projectors), odd
 projector counts (rows of 8, split rows of 2 x 64 and more), one and several
-buckets of the captured loop, the step kernel's clusters of 1 to 8 CTAs (few
-systems of many plane waves), and boxes that run the plane phases with radices
-taken at run time.  Converged solves (tr2 far below the production threshold) in
-FP64 against the oracle at the tolerance of the other parity tests (1e-10)."""
+buckets of the captured loop, the step kernel's CTAs of 256, 512 and 1,024 threads
+and clusters of four, and boxes that run the plane phases with radices taken at run
+time.  Converged solves (tr2 far below the production threshold) against the oracle
+at the tolerances of the other parity tests (1e-10, mixed form 1e-7)."""
 import dataclasses
 
 import numpy as np
@@ -16,27 +16,29 @@ from west_b200.system import SystemSpec, build_system, perturbations
 pytestmark = pytest.mark.gpu
 
 
-def _solve(s, dvg, graphs=True):
+def _solve(s, dvg, graphs=True, form="fp64"):
     from west_b200.wstat import ResponseOperator
     op = ResponseOperator(s, n_dfpt_maxiter=400, verbose=False)
     op.set_graphs(graphs)
+    op.set_precision(form)
     dng = np.zeros_like(dvg, order="F")
-    ierr = op.apply_operator(dvg.shape[1], dvg, dng, 1e-20, 1)
+    ierr = op.apply_operator(dvg.shape[1], dvg, dng, 1e-20 if form == "fp64" else 1e-14, 1)
     op.close()
     return dng, ierr
 
 
-def _check(s, m):
+def _check(s, m, form="fp64"):
+    tol = 1e-10 if form == "fp64" else 1e-7
     dvg = perturbations(s, m, seed=m)
     k = min(m, 2)                                   # the oracle takes the first and the last
     pick = [0, m - 1][:k]
     ref, rerr = O.apply_operator(s, np.asfortranarray(dvg[:, pick]), 1e-20, maxiter=400)
     assert (rerr == 0).all()
-    got, ierr = _solve(s, dvg)
+    got, ierr = _solve(s, dvg, form=form)
     assert (ierr == 0).all()
-    assert np.linalg.norm(got[:, pick] - ref) / np.linalg.norm(ref) < 1e-10
-    eager, _ = _solve(s, dvg, graphs=False)
-    assert np.linalg.norm(got - eager) / np.linalg.norm(eager) < 1e-10
+    assert np.linalg.norm(got[:, pick] - ref) / np.linalg.norm(ref) < tol
+    eager, _ = _solve(s, dvg, graphs=False, form=form)
+    assert np.linalg.norm(got - eager) / np.linalg.norm(eager) < tol
 
 
 @pytest.mark.parametrize("m", [1, 11, 21, 22, 43, 50])          # 3 bands: 3 to 150 systems
@@ -69,9 +71,77 @@ def test_reduction_of_many_projectors(tiny, total):
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-10
 
 
-@pytest.mark.parametrize("L,ecut,nr", [(13.0, 12.0, 32), (15.0, 20.0, 48), (17.0, 25.0, 60)])   # clusters of 2, 4, 8
-def test_step_clusters(L, ecut, nr):
-    _check(build_system(SystemSpec(L=L, ecutwfc=ecut, nr=nr, natoms=2, nbnd_occ=3, proj="s", seed=4), "cuda"), 2)
+# plane waves up to 1,024, up to 4,095, and more: one CTA of 256 or 512 threads, clusters of four
+_STEP_CELLS = [(13.0, 12.0, 32, 0, 1024), (15.0, 18.0, 45, 1025, 4095), (17.0, 25.0, 60, 4096, 10 ** 6)]
+
+
+def _step_cell(L, ecut, nr, lo, hi):
+    s = build_system(SystemSpec(L=L, ecutwfc=ecut, nr=nr, natoms=2, nbnd_occ=3, proj="s", seed=4), "cuda")
+    assert lo <= s.npw <= hi
+    return s
+
+
+@pytest.mark.parametrize("form", ["fp64", "mixed"])
+@pytest.mark.parametrize("m", [2, 23])                          # 6 systems, and 69: 1,024 threads in the last cell
+@pytest.mark.parametrize("cell", _STEP_CELLS)
+def test_step_shapes(cell, m, form):
+    _check(_step_cell(*cell), m, form)
+
+
+@pytest.mark.parametrize("form", ["fp64", "mixed"])
+@pytest.mark.parametrize("L,nr", [(25.0, 80), (30.0, 108)])     # clusters of 2 and 4 in FP64, 1 and 2 in FP32
+def test_step_clusters_of_large_cells(L, nr, form):
+    """66 systems, whose vectors pass L2 with one CTA each, against the same
+    perturbations one by one (clusters of four)."""
+    s = build_system(SystemSpec(L=L, ecutwfc=25.0, nr=nr, natoms=2, nbnd_occ=3, proj="s", seed=4), "cuda")
+    assert s.npw > 16000
+    dvg = perturbations(s, 22, seed=1)
+    got, ierr = _solve(s, dvg, form=form)
+    assert (ierr == 0).all()
+    for p in (0, 21):
+        one, _ = _solve(s, np.asfortranarray(dvg[:, p:p + 1]), form=form)
+        assert np.linalg.norm(got[:, p] - one[:, 0]) / np.linalg.norm(one) < (1e-10 if form == "fp64" else 1e-7)
+
+
+@pytest.mark.parametrize("form", ["fp64", "mixed"])
+@pytest.mark.parametrize("cell", _STEP_CELLS)
+def test_bits_do_not_depend_on_earlier_calls(cell, form):
+    """A call gives the same bits first on its context, after larger calls (whose
+    workspace its captured loop then has) and eagerly, and up to 64 systems through the
+    allocation-free entry point where they fit it."""
+    import ctypes
+    import torch
+    from west_b200 import lib as L
+    from west_b200.wstat import ResponseOperator
+    s = _step_cell(*cell)
+    dvg = perturbations(s, 43, seed=2)
+
+    def op():
+        o = ResponseOperator(s, verbose=False)
+        o.set_precision(form)
+        o.set_autotune(False)                                   # shapes tuned by time differ from context to context
+        return o
+
+    def run(o, m):
+        dng = np.zeros((s.npw, m), dtype=np.complex128, order="F")
+        o.apply_operator(m, np.asfortranarray(dvg[:, :m]), dng, 1e-10, 1)
+        return dng
+
+    grown, eager = op(), op()
+    eager.set_graphs(False)
+    run(grown, 43)
+    for m in (1, 22, 43, 1):
+        first = run(op(), m)
+        assert np.array_equal(run(grown, m), first), m
+        assert np.array_equal(run(eager, m), first), m
+    if form == "fp64":
+        o, dv = op(), torch.from_numpy(np.ascontiguousarray(dvg[:, :1].T)).cuda()
+        out = torch.zeros_like(dv)
+        ierr = ctypes.c_int(-1)
+        rc = L.load().wb_apply_operator_device_noalloc(o._ctx, 1, dv.data_ptr(), s.npw, out.data_ptr(), s.npw, 1e-10, 1,
+                                                       ctypes.addressof(ierr))
+        assert rc == 0 and ierr.value == 0
+        assert np.array_equal(out.cpu().numpy().T, run(op(), 1))
 
 
 @pytest.mark.parametrize("L,ecut,nr", [

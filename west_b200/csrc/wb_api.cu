@@ -619,7 +619,7 @@ bool graph_mode(const wb_ctx* c) { return c->use_graphs && c->prof == 0; }
 // A workspace of one bucket needs no SWITCH: WHILE { one PCG pass }, whose step
 // kernel counts the pass and sets the condition (two launches and a conditional
 // node less of about ten per pass, where a pass takes 50 us).
-constexpr int kMinBucketItems = 32;
+constexpr int kMinBucketItems = kBucketSystems / 2;
 
 template <class Pass>
 int capture_loop(wb_ctx* c, wb_ctx::LoopCache& cache, std::vector<const void*> key, double tr2, int cap,

@@ -228,6 +228,17 @@ void cg_prec_rho(const int* act, int nact, const double2* g, double2* P, const d
 // nact_host may be null (no host copy); nsys_dev, if given, overrides nsys
 void cg_compact(const unsigned char* conv, int nsys, int* act, int2* items, int* nact_dev, int* nact_host,
                 cudaStream_t s, const int* nsys_dev = nullptr);
+// The captured PCG loops have one branch per bucket of active systems: up to 64, 128,
+// 256, ... (wb_api.cu, capture_loop).  bucket_systems: the bound of the bucket that
+// serves n systems.  A captured launch is sized for that bound or, in the last bucket,
+// for the workspace's capacity, an eager one for the live count: all three have the
+// same bucket, so a launch shape that decides the order of a sum depends on it only.
+constexpr int kBucketSystems = 64;
+inline int bucket_systems(int n) {
+  int b = kBucketSystems;
+  while (b < n) b *= 2;
+  return b;
+}
 // Loop state a captured PCG pass hands to its step kernel (wb_la.cu, CgTail):
 // the active list it rebuilds and, with ctl, the WHILE condition it sets.
 struct CgLoop {

@@ -248,9 +248,9 @@ void gemm_tn(const double* W, long ldw, int M, const double* X, long ldx, const 
 // projectors q of D) of a row r and are summed in a fixed order, so that the
 // loads of a column are in flight together instead of one after the other.
 constexpr int kRedThreads = 512;
-// many columns fill the GPU by themselves and small blocks cost least (1,200
+// many columns (buckets above 256) fill the GPU by themselves and small blocks cost least (1,200
 // columns of 64 projectors: 17 us against 24); few need the width
-static int red_threads(int ncol) { return ncol >= 512 ? 128 : kRedThreads; }
+static int red_threads(int ncol) { return ncol > 256 ? 128 : kRedThreads; }
 template <class T, class F>
 WB_DEV void grouped_sum(T* out, T* scratch, int M, int n, F term) {  // out[r] = sum_{i < n} term(r, i)
   int rw = 32;
@@ -857,26 +857,36 @@ __global__ void __launch_bounds__(NT) k_cg_step(const int* act, const int* dn, i
   }
 }
 
-// CTAs per system.  Enough that few systems still cover the SMs (a slice keeps
-// 512 plane waves), and that the systems in flight, one CTA per SM in FP64 and
-// two in FP32, keep their four vectors in L2 between the passes: the 108^3
-// cell's FP64 vectors are 598 KB, 354 MB for 148 systems.  Measured per call
-// there: 4 CTAs 33 ms, 8 41, 1 41 in FP64; 8 CTAs 46 ms, 4 48, 1 68 in FP32; at
-// 64^3 (80 MB for 148 systems) 1 CTA 16.7 ms, 2 20.7.  One perturbation at 64^3,
-// 19 systems: 24 us a step with one CTA each, 13 with 4.
-static int cg_cluster(int nmax, int npw, int elem) {
-  const int ctas = elem == 16 ? sm_count() : 2 * sm_count();
+// Threads per CTA and CTAs per system.  The choice and with it the order of the sums
+// depends on the count's bucket alone (bucket_systems), not on the workspace's capacity
+// or on how many systems are left of a bucket, so that a call has the same bits
+// whatever ran on its context before, captured or not.  Measured on one B200, us a step:
+//   up to 64 systems, 512 threads: the slices' serial passes are the time.  64^3 (8,440
+//     plane waves) 24 systems FP64 12.8 with 4 CTAs, 16.9 with 2, 19.9 with 1; 64
+//     systems 17.0, 16.9 and 20.8 (4 CTAs of 1024 threads 25.6: two waves).  Below
+//     4,096 plane waves one CTA: 2,400 plane waves, 64 systems 8.8, with 4 CTAs 10.8.
+//   more systems, 1024 threads, one CTA per SM: the fewest CTAs per system with which
+//     the systems in flight keep their four vectors in 96 MB of L2 between the passes.
+//     2,048 systems FP64: 8,440 plane waves 437 with 1 CTA, 571 with 2; 16,900 1,085,
+//     1,010 with 2, 1,325 with 4; 37,387 2,506, 2,649 and 2,396 with 4.  FP32: 16,900 566
+//     with 1 and 642 with 2, 37,387 1,583 with 1, 1,373 with 2 and 1,604 with 4.
+struct CgShape {
+  int threads, ctas;
+};
+static CgShape cg_shape(int n, int npw, int elem) {
+  if (npw <= 1024) return {256, 1};
+  if (npw < 4096) return {512, 1};
+  const int systems = bucket_systems(n);
+  if (systems <= kBucketSystems) return {512, 4};
   int cs = 1;
-  while (cs < 8 && (long)nmax * 2 * cs <= ctas && 2 * cs * 512 <= npw) cs *= 2;
-  while (cs < 8 && 4.0 * elem * npw * (double)std::min(nmax, ctas / cs) > (cs > 1 && elem == 8 ? 50e6 : 96e6)) cs *= 2;
-  return cs;
+  while (cs < 8 && 4.0 * elem * npw * (double)std::min(systems, sm_count() / cs) > 96e6) cs *= 2;
+  return {1024, cs};
 }
 template <class C, int NT, int CS, class... A>
 static void cg_step_launch(int nact, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   // one CTA per system: a persistent grid, so that no more systems than fit L2 are in flight
-  const int resident = (sizeof(C) == 16 ? 1 : 2) * sm_count();
-  cfg.gridDim = dim3(CS == 1 ? std::min(nact, resident) : nact * CS);
+  cfg.gridDim = dim3(CS == 1 ? std::min(nact, sm_count() * (1024 / NT)) : nact * CS);
   cfg.blockDim = dim3(NT);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
@@ -901,39 +911,40 @@ static CgTail cg_tail(const CgLoop* l) {
   t.inner = l->inner;
   return t;
 }
+template <class C>
+static void cg_step_t(const int* act, int n, C* x, C* g, C* P, const C* T, const double* iprec, int nocc,
+                      double* rho_prev, unsigned char* conv, int iter, int maxiter, double tr2, const double* rel,
+                      double floor, int npw, long ld, cudaStream_t s, const int* dn, const int* iter_dev,
+                      const CgLoop* loop) {
+  if (n <= 0) return;
+  const CgShape sh = cg_shape(n, npw, sizeof(C));
+  auto go = [&](auto launch) {
+    launch(n, s, act, dn, n, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, tr2, rel, floor, npw,
+           ld, cg_tail(loop));
+  };
+#define WB_STEP(NT, CS) \
+  if (sh.threads == NT && sh.ctas == CS) return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<C, NT, CS>(m, q, a...); })
+  WB_STEP(256, 1);
+  WB_STEP(512, 1);
+  WB_STEP(512, 4);
+  WB_STEP(1024, 1);
+  WB_STEP(1024, 2);
+  WB_STEP(1024, 4);
+  WB_STEP(1024, 8);
+#undef WB_STEP
+}
 void cg_step(const int* act, int nact, double2* x, double2* g, double2* P, const double2* T, const double* iprec,
              int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double tr2, int npw, long ld,
              cudaStream_t s, const int* dn, const int* iter_dev, const CgLoop* loop) {
-  if (nact <= 0) return;
-  const double* rel = nullptr;
-  auto go = [&](auto launch) {
-    launch(nact, s, act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, tr2, rel, 0.0,
-           npw, ld, cg_tail(loop));
-  };
-  if (npw <= 1024) return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 256, 1>(m, q, a...); });
-  switch (cg_cluster(nact, npw, 16)) {
-    case 1: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 1>(m, q, a...); });
-    case 2: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 2>(m, q, a...); });
-    case 4: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 4>(m, q, a...); });
-    default: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<double2, 1024, 8>(m, q, a...); });
-  }
+  cg_step_t<double2>(act, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, maxiter, tr2, nullptr, 0.0, npw, ld, s,
+                     dn, iter_dev, loop);
 }
 void cg_step32(const int* act, int nact, float2* x, float2* g, float2* P, const float2* T, const double* iprec,
                int nocc, double* rho_prev, unsigned char* conv, int iter, int maxiter, double eta, const double* rel,
                double floor, int npw, long ld, cudaStream_t s, const int* dn, const int* iter_dev,
                const CgLoop* loop) {
-  if (nact <= 0) return;
-  auto go = [&](auto launch) {
-    launch(nact, s, act, dn, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, iter_dev, maxiter, eta, rel, floor,
-           npw, ld, cg_tail(loop));
-  };
-  if (npw <= 1024) return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 256, 1>(m, q, a...); });
-  switch (cg_cluster(nact, npw, 8)) {
-    case 1: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 1>(m, q, a...); });
-    case 2: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 2>(m, q, a...); });
-    case 4: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 4>(m, q, a...); });
-    default: return go([](int m, cudaStream_t q, auto... a) { cg_step_launch<float2, 512, 8>(m, q, a...); });
-  }
+  cg_step_t<float2>(act, nact, x, g, P, T, iprec, nocc, rho_prev, conv, iter, maxiter, eta, rel, floor, npw, ld, s, dn,
+                    iter_dev, loop);
 }
 
 // ---------------------------------------------------------------------------
