@@ -150,19 +150,20 @@ int wb_apply_operator_multi(int nctx, wb_ctx* const* ctx, const int* m, const do
                             double* const* dng, const int* ld_dng, double tr2, int iq, int* const* unconverged,
                             int on_device);
 
-/* Launch shapes chosen by the library's autotuner, which times the candidates
- * on the first batch of each form (FP64, mixed) on the batch's own buffers
- * before its PCG loop starts, then keeps them for the context. */
+/* Launch shapes.  The autotuner times those of the mixed form's tcgen05 GEMMs on
+ * the form's first batch, on the batch's own buffers before its PCG loop starts,
+ * and keeps them for the context; the FP64 form's follow from the sizes alone.
+ * Fields marked (fixed) are kept for callers compiled against them. */
 typedef struct wb_tuning {
   int autotune;              /* 1: tune on first use (default); 0: built-in shapes   */
-  int tuned_fp64;            /* 1 once the FP64 form was tuned                        */
+  int tuned_fp64;            /* 1 after the first FP64 batch with autotune on         */
   int tuned_mixed;           /* 1 once the mixed form was tuned                       */
-  int dmma_ctas_per_sm;      /* FP64 bra-ket split-K target, CTAs per SM (1, 2, 4)    */
+  int dmma_ctas_per_sm;      /* (fixed) FP64 bra-ket: CTAs per SM of the split rule, 4 */
   int tc_braket_ctas_per_sm; /* tcgen05 bra-ket split-K target, CTAs per SM (1..3)    */
   int tc_update_systems;     /* systems per CTA of the tcgen05 update (64, 128; 0 default) */
-  int plane_fused_fp64;      /* 1: one-pass fused plane kernel in the FP64 operator   */
-  int plane_fused_mixed;     /* 1: the same in the FP32 inner operator                */
-  int dmma_prefetch;         /* FP64 bra-ket: stages loaded ahead of the MMA (fixed: 2)  */
+  int plane_fused_fp64;      /* (fixed) 1: a box with compiled plane kernels           */
+  int plane_fused_mixed;     /* (fixed) the same                                      */
+  int dmma_prefetch;         /* (fixed) FP64 bra-ket: stages loaded ahead of the MMA, 2 */
   float tuning_ms;           /* host time spent tuning                                */
 } wb_tuning;
 int wb_get_tuning(const wb_ctx* ctx, wb_tuning* out);

@@ -260,7 +260,7 @@ size_t per_pert_bytes(const wb_ctx* c) {
          + stk * (size_t)c->npv                    // sticks (RHS / CG pairs / drho items)
          + sizeof(double2) * (size_t)c->nnr * 1    // dvbox + acc (one box per two perturbations each)
          + stk                                     // sticks2 (half per perturbation, rounded up)
-         + sizeof(double) * (size_t)c->nocc * c->nproj * 9  // GEMM partials and coefficients
+         + sizeof(double) * (size_t)c->nocc * c->nproj * 40  // GEMM partials and coefficients
          + 2 * sizeof(double2) * (size_t)c->npw;   // aux, input/output staging
 }
 
@@ -291,9 +291,9 @@ int ensure_workspace(wb_ctx* c, int mb, long ld_in, long ld_out) {
   bad |= c->sticks.ensure(stk1 * nitems) != 0;
   bad |= c->sticks2.ensure(stk1 * mp) != 0;
   bad |= c->acc.ensure(sizeof(double2) * (size_t)c->nnr * mp) != 0;
-  // all projectors or the bands alone, up to the tuner's largest target
-  bad |= c->part.ensure(sizeof(double) * std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw, 4),
-                                                   gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw, 4))) != 0;
+  // all projectors or the bands alone
+  bad |= c->part.ensure(sizeof(double) * std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw),
+                                                   gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw))) != 0;
   bad |= c->C.ensure(sizeof(double) * nsys * c->nproj) != 0;
   bad |= c->rho.ensure(sizeof(double) * nsys) != 0;
   bad |= c->conv.ensure(nsys + 16) != 0;
@@ -327,35 +327,6 @@ float time_ms(wb_ctx* c, F fn) {
     if (cudaEventElapsedTime(&ms, c->tev0, c->tev1) == cudaSuccess) best = std::min(best, ms);
   }
   return best;
-}
-
-// FP64 form: split-K target of the DMMA bra-ket (1, 2 or 4 CTAs per SM), timed
-// on this batch's still unused buffers (X zeroed; part and the active list are
-// rewritten by the batch afterwards).
-int autotune64(wb_ctx* c, int nsys) {
-  if (!c->tune.on || c->tune.done64) return WB_OK;
-  c->tune.done64 = 1;
-  const auto t0 = std::chrono::steady_clock::now();
-  cudaStream_t s = c->stream;
-  const int K = 2 * c->npw;
-  const long ld = c->npw;
-  const int M = c->kinetic_only ? c->nocc : c->nproj;
-  const double* W = c->W.as<double>() + (c->kinetic_only ? (size_t)c->nkb * K : 0);
-  WB_CU(cudaMemsetAsync(c->X.p, 0, sizeof(double2) * ld * nsys, s));
-  cg_reset(c->conv.as<unsigned char>(), nsys, s);
-  cg_compact(c->conv.as<unsigned char>(), nsys, c->act.as<int>(), c->items.as<int2>(), c->nact.as<int>(), nullptr, s);
-  float best = 3.4e38f;
-  for (int ctas : {1, 2, 4}) {
-    const int ns = gemm_tn_plan(M, nsys, K, ctas);
-    const float ms = time_ms(c, [&] {
-      gemm_tn(W, K, M, (const double*)c->X.p, 2 * ld, c->act.as<int>(), nsys, K, ns, c->part.as<double>(), s,
-              nullptr, ctas);
-    });
-    if (ms < best) { best = ms; c->tune.dmma_ctas = ctas; }
-  }
-  WB_CU(cudaGetLastError());
-  c->tune.ms += std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  return WB_OK;
 }
 
 // Mixed form: split-K target of the tcgen05 bra-ket (1..3 CTAs per SM) and systems
@@ -432,18 +403,17 @@ void apply_A(wb_ctx* c, const double2* Xv, double2* Tv, const int* cols, const i
   }
   // In a captured pass the bra-ket and its reduction, which need X alone, are a
   // second branch beside the local potential.
-  const int nsplit = gemm_tn_plan(M, n, K, c->tune.dmma_ctas);
+  const int nsplit = gemm_tn_plan(M, n, K);
   const bool side = dn && forked(c, n);
   const cudaStream_t sb = side ? fork_side(c) : s;
   {
     Stage g(c, WB_STAGE_GEMM_TN, 1, n);
-    gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, nsplit, c->part.as<double>(), sb, dn,
-            c->tune.dmma_ctas);
+    gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, nsplit, c->part.as<double>(), sb, dn);
   }
   {
     Stage g(c, WB_STAGE_GEMM_REDUCE, 1, n);
     gamma_reduce(c->part.as<double>(), nsplit, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(),
-                 nkb, c->alpha, c->C.as<double>(), sb, dn, K, c->tune.dmma_ctas);
+                 nkb, c->alpha, c->C.as<double>(), sb, dn, K);
   }
   if (c->kinetic_only) {
     Stage g(c, WB_STAGE_VLOC_ZFWD, 1, n);
@@ -881,9 +851,8 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
   c->stats.fft_boxes += mp + (long long)mb * npv;
   // 4. dvpsi <- -Pc dvpsi = -dvpsi + evc (evc^T dvpsi)  (dfpt_module.f90:346)
   const double* Wevc = c->W.as<double>() + (size_t)c->nkb * K;
-  int rc0 = autotune64(c, nsys);
-  if (rc0) return rc0;
-  const int nsplit = gemm_tn_plan(nocc, nsys, K, c->tune.dmma_ctas);
+  c->tune.done64 |= c->tune.on;  // nothing of the FP64 form is timed: the split plan is a rule
+  const int nsplit = gemm_tn_plan(nocc, nsys, K);
   {
     Stage g(c, WB_STAGE_OTHER, 4, nsys);
     gemm_tn(Wevc, K, nocc, (const double*)B, 2 * ld, nullptr, nsys, K, nsplit, c->part.as<double>(), s);
@@ -1362,8 +1331,8 @@ int wb_get_tuning(const wb_ctx* c, wb_tuning* out) {
   out->autotune = c->tune.on;
   out->tuned_fp64 = c->tune.done64;
   out->tuned_mixed = c->tune.done32;
-  out->dmma_ctas_per_sm = c->tune.dmma_ctas;
-  out->dmma_prefetch = kDmmaAhead;
+  out->dmma_ctas_per_sm = 4;
+  out->dmma_prefetch = 2;
   out->tc_braket_ctas_per_sm = c->tune.umma_ctas;
   out->tc_update_systems = c->tune.update_nj;
   out->plane_fused_fp64 = out->plane_fused_mixed = c->rt ? 0 : 1;
@@ -1443,8 +1412,6 @@ struct Carve {
   }
 };
 
-constexpr int kNoallocCtas = 2;  // the built-in split target
-
 struct NoallocWs {
   FftArgs fa;  // the context's, or with its sticks unpadded
   double2 *aux, *dvbox, *B, *X, *G, *T, *sticks, *sticks2, *acc;
@@ -1481,8 +1448,8 @@ void noalloc_layout(const wb_ctx* c, int mb, int level, Carve& cv, NoallocWs& w)
   w.sticks = cv.take<double2>(stk1 * nitems);
   w.sticks2 = cv.take<double2>(stk1 * mp);
   w.acc = cv.take<double2>((size_t)c->nnr * mp);
-  w.part = cv.take<double>(plan ? std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw, kNoallocCtas),
-                                           gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw, kNoallocCtas))
+  w.part = cv.take<double>(plan ? std::max(gemm_tn_part_doubles(c->nproj, (int)nsys, 2 * c->npw),
+                                           gemm_tn_part_doubles(c->nocc, (int)nsys, 2 * c->npw))
                                 : (size_t)w.nsplit * nsys * c->nproj);
   w.C = cv.take<double>(nsys * c->nproj);
   w.rho = cv.take<double>(nsys);
@@ -1526,7 +1493,7 @@ void noalloc_apply_A(wb_ctx* c, const NoallocWs& w, const double2* Xv, double2* 
     fft_plane_vloc(w.fa, w.sticks, nit, c->vs.as<double>());
     fft_zfwd_hpsi(w.fa, w.sticks, items, nit, Xv, Tv, ld, c->g2kin.as<double>(), w.ecol);
   }
-  const int ns = w.plan ? gemm_tn_plan(M, n, K, kNoallocCtas) : w.nsplit;
+  const int ns = w.plan ? gemm_tn_plan(M, n, K) : w.nsplit;
   gemm_tn(Wsub, K, M, (const double*)Xv, 2 * ld, cols, n, K, ns, w.part, s);
   gamma_reduce(w.part, ns, M, n, Wsub, K, (const double*)Xv, 2 * ld, cols, c->D.as<double>(), nkb, c->alpha,
                w.C, s);
@@ -1551,7 +1518,7 @@ int noalloc_run(wb_ctx* c, const NoallocWs& w, int mb, const double2* dvg, long 
   fft_plane_rhs(w.fa, c->evcr.as<double2>(), w.dvbox, npv, mb, w.sticks);
   fft_zfwd_store(w.fa, w.sticks, w.items_pk, mb * npv, w.B, ld);
   const double* Wevc = c->W.as<double>() + (size_t)c->nkb * K;
-  const int ns = w.plan ? gemm_tn_plan(nocc, nsys, K, kNoallocCtas) : w.nsplit;
+  const int ns = w.plan ? gemm_tn_plan(nocc, nsys, K) : w.nsplit;
   gemm_tn(Wevc, K, nocc, (const double*)w.B, 2 * ld, nullptr, nsys, K, ns, w.part, s);
   gamma_reduce(w.part, ns, nocc, nsys, Wevc, K, (const double*)w.B, 2 * ld, nullptr, nullptr, 0, 1.0, w.C, s);
   gemm_nn(Wevc, K, nocc, w.C, (double*)w.B, 2 * ld, nullptr, nsys, K, -1.0, s);

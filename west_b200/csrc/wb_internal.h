@@ -152,6 +152,17 @@ void fft_plane_drho(const FftArgs& f, const double2* dsticks, const double2* evc
 
 // ---- dense kernels (wb_la.cu) ----
 // part[s][j][r] = sum_{k in split s} W[r*ldw + k] * X[col(j)*ldx + k]
+// The captured PCG loops have one branch per bucket of active systems: up to 64, 128,
+// 256, ... (wb_api.cu, capture_loop).  bucket_systems: the bound of the bucket that
+// serves n systems.  A captured launch is sized for that bound or, in the last bucket,
+// for the workspace's capacity, an eager one for the live count: all three have the
+// same bucket, so a launch shape that decides the order of a sum depends on it only.
+constexpr int kBucketSystems = 64;
+inline int bucket_systems(int n) {
+  int b = kBucketSystems;
+  while (b < n) b *= 2;
+  return b;
+}
 // Split-K plans of the bra-ket GEMMs, host and device: a graph replay sizes its
 // split grid for the largest plan and every CTA derives the plan of the device
 // column count itself, so both paths split the same count the same way.
@@ -167,39 +178,51 @@ __host__ __device__ inline int gemm_tn_splits(int M, int ncol, int K, int ctas_p
 }
 // k's of one split: a multiple of the pair width and of 16
 __host__ __device__ inline int gemm_tn_chunk(int K, int nsplit) { return ((K + nsplit - 1) / nsplit + 15) / 16 * 16; }
-// gemm_tn_plan: splits of the PCG's bra-kets.  Up to kDmmaSmall columns the 32 x
-// 32 tile runs and a CTA's serial chain is the time: about two CTAs per SM, at
-// least 128 k each.  Above, tiles of 64 columns and 64 rows (112 where there are
-// more): about ctas_per_sm CTAs per SM over the whole grid, at least 256 k each.
-constexpr int kDmmaAhead = 2;   // stages of operands a CTA loads ahead of its MMAs, at least
-constexpr int kDmmaSmall = 64;
-__host__ __device__ inline int gemm_tn_plan(int M, int ncol, int K, int ctas_per_sm) {
-  const bool small = ncol <= kDmmaSmall;
-  const int tr = small ? 32 : M > 64 ? 112 : 64, tj = small ? 32 : 64;
-  const int tiles = ((M + tr - 1) / tr) * ((ncol + tj - 1) / tj);
-  const int target = small ? 2 * 148 : 148 * ctas_per_sm;
-  int ns = target / (tiles > 0 ? tiles : 1);  // not over the target: a few CTAs more would be a whole wave
-  const int maxs = K / (small ? 128 : 256);
-  if (ns > maxs) ns = maxs;
-  if (ns < 1) ns = 1;
-  return ns;
+// gemm_tn_plan: splits of the PCG's bra-kets.  At most 896 k each (32 splits of a long K),
+// because a split's k's are one chain of additions per warp and its error grows with the
+// root of the chain's length; at least 384, below which the partial sums cost more than
+// the rounds saved, or 192 where the grid would otherwise leave half of the GPU's CTA
+// slots empty and a CTA's latency is the time.  Between these bounds four CTAs per SM,
+// then the first count of eight whose last round over 148 SMs is at least 95% full.
+// Bra-ket and reduction over 460 shapes (8 to 2,048 columns, 16 to 288 rows, K from 400 to
+// 74,774) stay within 1.9% of the best split on average, 9% at the 97th percentile.
+__host__ __device__ inline int gemm_tn_plan(int M, int ncol, int K) {
+  int tiles = ((M + 31) / 32) * ((ncol + 31) / 32);
+  if (tiles < 1) tiles = 1;
+  int lo = (K + 895) / 896, hi = K / 384;
+  if (lo > 32) lo = 32;
+  if (lo < 1) lo = 1;
+  if (hi < lo) hi = lo;
+  if (tiles * hi < 296) {
+    const int fill = 296 / tiles < K / 192 ? 296 / tiles : K / 192;
+    if (hi < fill) hi = fill;
+  }
+  int ns = 592 / tiles;
+  if (ns < lo) ns = lo;
+  if (ns > hi) ns = hi;
+  int best = ns;
+  long best_ctas = 0, best_rounds = 0;
+  for (int t = ns; t < ns + 8 && t <= hi; ++t) {
+    const long ctas = (long)tiles * t, rounds = (ctas + 147) / 148;
+    if (rounds * 148 * 20 <= ctas * 21) return t;
+    if (!best_ctas || rounds * best_ctas < best_rounds * ctas) { best = t; best_ctas = ctas; best_rounds = rounds; }
+  }
+  return best;
 }
-// the largest plan of any count up to ncol that runs the same tile
-__host__ __device__ inline int gemm_tn_plan_max(int M, int ncol, int K, int ctas_per_sm) {
-  return gemm_tn_plan(M, ncol <= kDmmaSmall ? 1 : kDmmaSmall + 1, K, ctas_per_sm);
-}
-// part doubles for any column count up to nsys and any target up to ctas_max
-size_t gemm_tn_part_doubles(int M, int nsys, int K, int ctas_max);
-// with dn, ctas selects the device plan (nsplit is then ignored)
+// the largest plan of any count that a captured launch of bound ncol serves
+int gemm_tn_plan_max(int M, int ncol, int K);
+// part doubles for any column count up to nsys
+size_t gemm_tn_part_doubles(int M, int nsys, int K);
+// with dn the kernel takes the plan of the device count (nsplit is then ignored)
 void gemm_tn(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol, int K,
-             int nsplit, double* part, cudaStream_t s, const int* dn = nullptr, int ctas = 2);
+             int nsplit, double* part, cudaStream_t s, const int* dn = nullptr);
 // opts the GEMM kernels into their shared memory on the current device
 void la_setup();
 // S = 2 sum_s part - W0 X0 (Gamma bra-ket, glbrak.f90:39-40), then
 // C[j][r] = sum_{r'<nkb} D[r][r'] S[j][r'] for r < nkb, alpha S[j][r] otherwise
 void gamma_reduce(const double* part, int nsplit, int M, int ncol, const double* W, long ldw, const double* X,
                   long ldx, const int* cols, const double* D, int nkb, double alpha, double* C, cudaStream_t s,
-                  const int* dn = nullptr, int K = 0, int ctas = 0);
+                  const int* dn = nullptr, int K = 0);
 // Y[col(j)] = beta Y[col(j)] + W C[j]  over K real rows
 void gemm_nn(const double* W, long ldw, int M, const double* C, double* Y, long ldy, const int* cols, int ncol,
              int K, double beta, cudaStream_t s, const int* dn = nullptr);
@@ -228,17 +251,6 @@ void cg_prec_rho(const int* act, int nact, const double2* g, double2* P, const d
 // nact_host may be null (no host copy); nsys_dev, if given, overrides nsys
 void cg_compact(const unsigned char* conv, int nsys, int* act, int2* items, int* nact_dev, int* nact_host,
                 cudaStream_t s, const int* nsys_dev = nullptr);
-// The captured PCG loops have one branch per bucket of active systems: up to 64, 128,
-// 256, ... (wb_api.cu, capture_loop).  bucket_systems: the bound of the bucket that
-// serves n systems.  A captured launch is sized for that bound or, in the last bucket,
-// for the workspace's capacity, an eager one for the live count: all three have the
-// same bucket, so a launch shape that decides the order of a sum depends on it only.
-constexpr int kBucketSystems = 64;
-inline int bucket_systems(int n) {
-  int b = kBucketSystems;
-  while (b < n) b *= 2;
-  return b;
-}
 // Loop state a captured PCG pass hands to its step kernel (wb_la.cu, CgTail):
 // the active list it rebuilds and, with ctl, the WHILE condition it sets.
 struct CgLoop {

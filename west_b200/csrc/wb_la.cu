@@ -30,17 +30,11 @@ WB_DEV void dmma(double& d0, double& d1, double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// cp.async of 16 or (rows that are not 16-byte aligned) twice 8 bytes; zeros
+// cp.async of 16 bytes (a pair of k: every operand is a column of double2) or 8; zeros
 // when !ok.  Copies are committed in groups, one per stage of a ring.
-WB_DEV void cp_pair(double* smem, const double* gmem, bool ok, bool al16) {
+WB_DEV void cp_pair(double* smem, const double* gmem, bool ok) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  if (al16) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0) : "memory");
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s + 8), "l"(gmem + 1), "r"(ok ? 8 : 0)
-                 : "memory");
-  }
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
 }
 WB_DEV void cp_one(double* smem, const double* gmem, bool ok) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -52,53 +46,43 @@ WB_DEV void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "
 
 // ---------------------------------------------------------------------------
 // part[s][j][r] = sum_{k in split s} W[r][k] X[col j][k]        (A^T B, split K)
-// A CTA of four warps takes TR rows r x TJ columns j; stages of KS k's of both
-// operands stream through a ring of ST buffers in shared memory by cp.async, so
-// a CTA has (ST - 1) stages in flight whatever its warps do.  Rows of KS + 4
-// doubles put the fragments of a half-warp (4 rows x 4 k) on distinct banks.
-//   64 x 64 (warps 2 x 2 of 32 x 32): the throughput form up to 64 rows; 16
-//     wavefronts per 64 cycles of DMMA and 0.125 bytes per flop from L2.  64 rows,
-//     1,200 columns, K = 16,880: 26 TFLOP/s of the pipe's 36.9 (16 before, with
-//     32 x 32 tiles whose warps read their operands from global memory).
-//   112 x 64 (each warp 112 x 16): more rows, split evenly over tiles (208 rows as
-//     2 x 104), so that X is read once per 112 rows: 208 rows, 160 columns, K =
-//     74,774: 21 TFLOP/s (14 before, 18 with 64 x 64 tiles).
-//   small tile (32 x 32, the four warps interleave k and are summed at the end,
-//     KS = 64): few columns, where the time is the latency of one CTA's chain.
-// K is even and a stage reads pairs of k; al16: rows are 16-byte aligned.
+// A CTA takes 32 rows r x 32 columns j; its four warps interleave k and are summed at
+// the end.  Stages of 32 k's of both operands stream through a ring of three buffers
+// in shared memory by cp.async, so a CTA has two stages in flight whatever its warps
+// do, and four CTAs fit an SM.  Rows of 36 doubles put the fragments of a half-warp
+// (4 rows x 4 k) on distinct banks.  K is even and a stage reads pairs of k.
+// One tile for every size.  Bound by the FP64 tensor pipe (36.9 TFLOP/s) and its own
+// latency.  Against two larger ones with a warp per k, us and TFLOP/s: 64 rows, 2,048
+// columns, K = 16,880 154 and 29 (64 x 64: 142); 112 rows, 384 columns, K = 33,800 114
+// and 25 (112 x 64: 97), 208 rows, 384 columns, K = 74,774 413 and 29 (112 x 64: 416); but
+// 80 rows, 256 columns, K = 4,800 15 (112 x 64: 34), 32 rows, 2,048 columns, K = 16,880 83
+// (64 x 64: 140).  Their chains of additions are four times as long: error against sums
+// in extended precision 1.4e-15 and 1.9e-15 at the first and third size, here 5.2e-16
+// and 8.6e-16.
 // ---------------------------------------------------------------------------
-template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
-struct TnTile {
-  static constexpr int LD = KS + 4, ROWS = TR + TJ, STAGE = ROWS * LD;
-  static constexpr int RG = TR / WR / 8, JG = TJ / WJ / 8;
-  static constexpr int SMEM = (int)sizeof(double) * (STAGE * ST > WK * TR * TJ ? STAGE * ST : WK * TR * TJ);
-  static_assert(WR * WJ * WK == 4, "four warps");
-};
+constexpr int TN_T = 32, TN_K = 32, TN_ST = 3, TN_LD = TN_K + 4, TN_STAGE = 2 * TN_T * TN_LD;
+constexpr int TN_SMEM = (int)sizeof(double) * TN_STAGE * TN_ST;
+static_assert(TN_STAGE * TN_ST >= 4 * TN_T * TN_T, "the ring holds the four warps' sums");
 
-template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
-__global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ W, long ldw, int M,
-                                                 const double* __restrict__ X, long ldx,
-                                                 const int* __restrict__ cols, int ncol_host, const int* dn, int K,
-                                                 int kchunk, int ctas, int trows, int al16,
-                                                 double* __restrict__ part) {
-  using G = TnTile<TR, TJ, WR, WJ, WK, KS, ST>;
-  constexpr int LD = G::LD, RG = G::RG, JG = G::JG;
+__global__ void __launch_bounds__(128, 4) k_gemm_tn(const double* __restrict__ W, long ldw, int M,
+                                                    const double* __restrict__ X, long ldx,
+                                                    const int* __restrict__ cols, int ncol_host, const int* dn, int K,
+                                                    int kchunk, int trows, double* __restrict__ part) {
   extern __shared__ __align__(16) double tn_sm[];
   const int ncol = dev_count(dn, ncol_host);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lr = lane >> 2, lk = lane & 3;
-  const int r0 = blockIdx.x * trows, j0 = blockIdx.y * TJ, split = blockIdx.z;
+  const int r0 = blockIdx.x * trows, j0 = blockIdx.y * TN_T, split = blockIdx.z;
   const int rend = min(M, r0 + trows);
   if (j0 >= ncol) return;
   if (dn) {  // the split plan of this column count
-    const int ns = gemm_tn_plan(M, ncol, K, ctas);
+    const int ns = gemm_tn_plan(M, ncol, K);
     if (split >= ns) return;
     kchunk = gemm_tn_chunk(K, ns);
   }
   const int kb = split * kchunk, ke = min(K, kb + kchunk);
-  // copies: KS/2 pairs of k per row; a thread's pair index is fixed, its rows step
-  constexpr int PR = KS / 2, RSTEP = 128 / PR, NROW = G::ROWS / RSTEP;
-  static_assert(128 % PR == 0 && G::ROWS % RSTEP == 0, "copy shape");
+  // copies: TN_K/2 pairs of k per row; a thread's pair index is fixed, its rows step
+  constexpr int PR = TN_K / 2, RSTEP = 128 / PR, NROW = 2 * TN_T / RSTEP;
   const int kp = (tid % PR) * 2, row0 = tid / PR;
   const double* src[NROW];
   unsigned okm = 0;
@@ -106,210 +90,255 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ W, l
   for (int i = 0; i < NROW; ++i) {
     const int row = row0 + i * RSTEP;
     src[i] = W;
-    if (row < TR) {
+    if (row < TN_T) {
       const int r = r0 + row;
       if (r < rend) { src[i] = W + (long)r * ldw; okm |= 1u << i; }
     } else {
-      const int j = j0 + row - TR;
+      const int j = j0 + row - TN_T;
       if (j < ncol) { src[i] = X + (long)(cols ? cols[j] : j) * ldx; okm |= 1u << i; }
     }
   }
   auto fetch = [&](int st, int k0) {
-    double* d = tn_sm + st * G::STAGE + row0 * LD + kp;
+    double* d = tn_sm + st * TN_STAGE + row0 * TN_LD + kp;
     const int k = k0 + kp;
     const bool kok = k < ke;
 #pragma unroll
     for (int i = 0; i < NROW; ++i)
-      cp_pair(d + i * RSTEP * LD, src[i] + (kok ? k : 0), kok && (okm >> i & 1u), al16 != 0);
+      cp_pair(d + i * RSTEP * TN_LD, src[i] + (kok ? k : 0), kok && (okm >> i & 1u));
   };
-  const int wk = warp % WK, wj = warp / WK % WJ, wr = warp / WK / WJ;
-  const int rb = wr * (TR / WR), jb = wj * (TJ / WJ);
-  // fragments of eight rows or columns beyond M or ncol are skipped, warp-uniformly
-  const int nr = min(RG, max(0, (rend - r0 - rb + 7) / 8)), nj = min(JG, max(0, (ncol - j0 - jb + 7) / 8));
-  double acc[RG][JG][2];
+  // fragments of eight rows or columns beyond M or ncol are skipped, CTA-uniformly
+  const int nr = (rend - r0 + 7) / 8, nj = min(4, (ncol - j0 + 7) / 8);
+  double acc[4][4][2];
 #pragma unroll
-  for (int a = 0; a < RG; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < JG; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 #pragma unroll
-  for (int st = 0; st < ST - 1; ++st) {
-    if (kb + st * KS < ke) fetch(st, kb + st * KS);
+  for (int st = 0; st < TN_ST - 1; ++st) {
+    if (kb + st * TN_K < ke) fetch(st, kb + st * TN_K);
     cp_commit();
   }
   int st = 0;
-  for (int k0 = kb; k0 < ke; k0 += KS) {
-    cp_wait<ST - 2>();
-    __syncthreads();
-    const int kn = k0 + (ST - 1) * KS;
-    if (kn < ke) fetch(st == 0 ? ST - 1 : st - 1, kn);
-    cp_commit();
-    const double* sw = tn_sm + st * G::STAGE + (rb + lr) * LD + wk * 4 + lk;
-    const double* sx = tn_sm + st * G::STAGE + (TR + jb + lr) * LD + wk * 4 + lk;
-    if (nr >= RG - 1 && nj == JG) {  // at most one fragment of zero rows
+  for (int k0 = kb; k0 < ke; k0 += TN_K) {
+    cp_wait<TN_ST - 2>();
+    __syncthreads();  // the stage is here, and the last one is read by every warp
+    const double* sw = tn_sm + st * TN_STAGE + lr * TN_LD + warp * 4 + lk;
+    const double* sx = sw + TN_T * TN_LD;
+    if (nr >= 3 && nj == 4) {  // at most one fragment of zero rows
 #pragma unroll
-      for (int kk = 0; kk < KS; kk += 4 * WK) {
-        double av[RG], bv[JG];
+      for (int kk = 0; kk < TN_K; kk += 16) {
+        double av[4], bv[4];
 #pragma unroll
-        for (int i = 0; i < RG; ++i) av[i] = sw[i * 8 * LD + kk];
+        for (int i = 0; i < 4; ++i) {
+          av[i] = sw[i * 8 * TN_LD + kk];
+          bv[i] = sx[i * 8 * TN_LD + kk];
+        }
 #pragma unroll
-        for (int i = 0; i < JG; ++i) bv[i] = sx[i * 8 * LD + kk];
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int a = 0; a < RG; ++a)
-#pragma unroll
-          for (int b = 0; b < JG; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
+          for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
       }
-    } else if (nr > 0 && nj > 0) {
+    } else {
 #pragma unroll
-      for (int kk = 0; kk < KS; kk += 4 * WK) {
-        double bv[JG];
+      for (int kk = 0; kk < TN_K; kk += 16) {
+        double bv[4];
 #pragma unroll
-        for (int i = 0; i < JG; ++i) bv[i] = sx[i * 8 * LD + kk];
+        for (int i = 0; i < 4; ++i) bv[i] = sx[i * 8 * TN_LD + kk];
 #pragma unroll
-        for (int a = 0; a < RG; ++a)
+        for (int a = 0; a < 4; ++a)
           if (a < nr) {
-            const double av = sw[a * 8 * LD + kk];
+            const double av = sw[a * 8 * TN_LD + kk];
 #pragma unroll
-            for (int b = 0; b < JG; ++b)
+            for (int b = 0; b < 4; ++b)
               if (b < nj) dmma(acc[a][b][0], acc[a][b][1], av, bv[b]);
           }
       }
     }
-    st = st == ST - 1 ? 0 : st + 1;
+    const int kn = k0 + (TN_ST - 1) * TN_K;
+    if (kn < ke) fetch(st == 0 ? TN_ST - 1 : st - 1, kn);
+    cp_commit();
+    st = st == TN_ST - 1 ? 0 : st + 1;
   }
   cp_wait<0>();
-  if constexpr (WK == 1) {
+  __syncthreads();  // the ring becomes the warps' sums, [warp][j][r]
+  double* red = tn_sm + warp * TN_T * TN_T;
 #pragma unroll
-    for (int b = 0; b < JG; ++b)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = j0 + jb + b * 8 + 2 * lk + h;
-        if (j >= ncol) continue;
-        double* o = part + ((long)split * ncol + j) * M + r0 + rb + lr;
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
-        for (int a = 0; a < RG; ++a)
-          if (r0 + rb + a * 8 + lr < rend) o[a * 8] = acc[a][b][h];
-      }
-  } else {
-    static_assert(WK == 1 || (WR == 1 && WJ == 1), "k-interleaved warps share one tile");
-    __syncthreads();  // the ring becomes the warps' sums, [warp][j][r]
-    double* red = tn_sm + wk * TR * TJ;
+      for (int h = 0; h < 2; ++h) red[(b * 8 + 2 * lk + h) * TN_T + a * 8 + lr] = acc[a][b][h];
+  __syncthreads();
+  for (int e = tid; e < TN_T * TN_T; e += 128) {
+    const int r = r0 + e % TN_T, j = j0 + e / TN_T;
+    if (r >= rend || j >= ncol) continue;
+    double sum = 0.0;
 #pragma unroll
-    for (int a = 0; a < RG; ++a)
-#pragma unroll
-      for (int b = 0; b < JG; ++b)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) red[(b * 8 + 2 * lk + h) * TR + a * 8 + lr] = acc[a][b][h];
-    __syncthreads();
-    for (int e = tid; e < TR * TJ; e += 128) {
-      const int r = r0 + e % TR, j = j0 + e / TR;
-      if (r >= rend || j >= ncol) continue;
-      double sum = 0.0;
-#pragma unroll
-      for (int w = 0; w < WK; ++w) sum += tn_sm[w * TR * TJ + e];
-      part[((long)split * ncol + j) * M + r] = sum;
-    }
+    for (int w = 0; w < 4; ++w) sum += tn_sm[w * TN_T * TN_T + e];
+    part[((long)split * ncol + j) * M + r] = sum;
   }
 }
 
-size_t gemm_tn_part_doubles(int M, int nsys, int K, int ctas_max) {
+size_t gemm_tn_part_doubles(int M, int nsys, int K) {
   size_t best = 0;
-  for (int t = 1; t <= (nsys + 31) / 32; ++t) {
+  for (int t = 1; t <= (nsys + 31) / 32; ++t) {  // the plan changes with the column tiles
     const int n = std::min(nsys, t * 32);
-    for (int c = 1; c <= ctas_max; ++c) best = std::max(best, (size_t)gemm_tn_plan(M, n, K, c) * n * M);
+    best = std::max(best, (size_t)gemm_tn_plan(M, n, K) * n * M);
   }
   return best;
 }
-
-template <int TR, int TJ, int WR, int WJ, int WK, int KS, int ST>
-static void gemm_tn_launch(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol,
-                           int K, int nsplit, double* part, cudaStream_t s, const int* dn, int ctas, int al16) {
-  constexpr int SM = TnTile<TR, TJ, WR, WJ, WK, KS, ST>::SMEM;
-  auto k = k_gemm_tn<TR, TJ, WR, WJ, WK, KS, ST>;
-  const int tiles = (M + TR - 1) / TR, trows = ((M + tiles - 1) / tiles + 7) / 8 * 8;
-  dim3 grid(tiles, (ncol + TJ - 1) / TJ, nsplit);
-  k<<<grid, 128, SM, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, gemm_tn_chunk(K, nsplit), ctas, trows, al16, part);
+int gemm_tn_plan_max(int M, int ncol, int K) {
+  const int first = bucket_systems(ncol) == kBucketSystems ? 1 : bucket_systems(ncol) / 2 + 1;
+  int best = 1;
+  for (int t = (first + 31) / 32; t <= (ncol + 31) / 32; ++t) best = std::max(best, gemm_tn_plan(M, t * 32, K));
+  return best;
 }
+
 void gemm_tn(const double* W, long ldw, int M, const double* X, long ldx, const int* cols, int ncol, int K,
-             int nsplit, double* part, cudaStream_t s, const int* dn, int ctas) {
+             int nsplit, double* part, cudaStream_t s, const int* dn) {
   if (ncol <= 0 || M <= 0) return;
-  const int al16 = ldw % 2 == 0 && ldx % 2 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)X % 16 == 0;
-  // with dn the kernel follows the bound ncol, as gemm_tn_plan does the count: a
-  // graph bucket lies on one side of kDmmaSmall with every count it serves
-  if (dn) nsplit = gemm_tn_plan_max(M, ncol, K, ctas);
-  if (ncol <= kDmmaSmall)
-    gemm_tn_launch<32, 32, 1, 1, 4, 64, 3>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
-  else if (M > 64)
-    gemm_tn_launch<112, 64, 1, 4, 1, 16, 3>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
-  else
-    gemm_tn_launch<64, 64, 2, 2, 1, 16, 4>(W, ldw, M, X, ldx, cols, ncol, K, nsplit, part, s, dn, ctas, al16);
+  if (dn) nsplit = gemm_tn_plan_max(M, ncol, K);
+  const int tiles = (M + TN_T - 1) / TN_T, trows = ((M + tiles - 1) / tiles + 7) / 8 * 8;
+  dim3 grid(tiles, (ncol + TN_T - 1) / TN_T, nsplit);
+  k_gemm_tn<<<grid, 128, TN_SMEM, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, gemm_tn_chunk(K, nsplit), trows, part);
 }
 
-// One CTA per column; NG groups of threads share out the splits (then the
-// projectors q of D) of a row r and are summed in a fixed order, so that the
-// loads of a column are in flight together instead of one after the other.
-constexpr int kRedThreads = 512;
-// many columns (buckets above 256) fill the GPU by themselves and small blocks cost least (1,200
-// columns of 64 projectors: 17 us against 24); few need the width
-static int red_threads(int ncol) { return ncol > 256 ? 128 : kRedThreads; }
-template <class T, class F>
-WB_DEV void grouped_sum(T* out, T* scratch, int M, int n, F term) {  // out[r] = sum_{i < n} term(r, i)
-  int rw = 32;
-  while (rw < M && rw < (int)blockDim.x) rw *= 2;
-  const int ng = blockDim.x / rw, g = threadIdx.x / rw;
-  for (int r0 = 0; r0 < M; r0 += rw) {
-    const int r = r0 + threadIdx.x % rw;
-    T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    if (r < M) {
-      int i = g;
-      for (; i + 3 * ng < n; i += 4 * ng) {
-        s0 += term(r, i);
-        s1 += term(r, i + ng);
-        s2 += term(r, i + 2 * ng);
-        s3 += term(r, i + 3 * ng);
-      }
-      for (; i < n; i += ng) s0 += term(r, i);
-    }
-    scratch[threadIdx.x] = (s0 + s1) + (s2 + s3);
-    __syncthreads();
-    if (g == 0 && r < M) {
-      T t = 0;
-      for (int q = 0; q < ng; ++q) t += scratch[q * rw + threadIdx.x];
-      out[r] = t;
-    }
-    __syncthreads();
+// The reductions of the bra-kets, FP64 (split plan of k_gemm_tn) and FP32 (of the
+// tcgen05 bra-ket): S = 2 sum_s part - W0 X0, then C = D S for the projectors, alpha S
+// for the bands.
+template <class T>
+WB_DEV int red_splits(int nsplit, const int* dn, int M, int ncol, int K, int ctas) {
+  if constexpr (sizeof(T) == 8) {
+    return dn ? gemm_tn_plan(M, ncol, K) : nsplit;
+  } else {
+    int per;
+    if (dn && ctas > 0) umma_braket_plan(ncol, K, &nsplit, &per, ctas);
+    return nsplit;
   }
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_gamma_reduce(const double* __restrict__ part, int nsplit, int M,
-                                                      int ncol_host, const int* dn, const double* __restrict__ W,
-                                                      long ldw, const double* __restrict__ X, long ldx,
-                                                      const int* __restrict__ cols, const double* __restrict__ D,
-                                                      int nkb, double alpha, double* __restrict__ C, int K,
-                                                      int ctas) {
-  extern __shared__ double S[];
-  __shared__ double scratch[kRedThreads];
+// One CTA per column.  GROUPS (up to 512 columns): groups of threads share out a row's
+// splits (eight partial sums each), then a row's projectors q of D, and are summed in
+// order through shared memory, since the time is the chain of loads; without it a thread
+// has a row to itself (four partial sums), and more columns are in flight.  us, with
+// groups and without: 64 rows, 64 columns of 74 splits 6.6 and 17, 2,048 columns of 19
+// splits 17 and 11; 208 rows, 64 columns of 42 splits 11 and 19, 2,048 columns 47 and 36.
+// Several columns per CTA, to read D less often, lost to the longer chain: 64 rows, 1,024
+// columns 7 with one, 13 with two, 15 with four.
+template <class T, int NT, bool GROUPS>
+__global__ void __launch_bounds__(NT) k_gamma_reduce(const T* __restrict__ part, int nsplit, int M, int ncol_host,
+                                                     const int* dn, const T* __restrict__ W, long ldw,
+                                                     const T* __restrict__ X, long ldx, const int* __restrict__ cols,
+                                                     const T* __restrict__ D, int nkb, T alpha, T* __restrict__ C,
+                                                     int K, int ctas) {
+  extern __shared__ __align__(16) unsigned char red_sm[];
+  T* S = reinterpret_cast<T*>(red_sm);
   const int ncol = dev_count(dn, ncol_host);
   const int j = blockIdx.x;
   if (j >= ncol) return;
-  if (dn && ctas > 0) nsplit = gemm_tn_plan(M, ncol, K, ctas);
+  nsplit = red_splits<T>(nsplit, dn, M, ncol, K, ctas);
   const int col = cols ? cols[j] : j;
-  const double x0 = X[(long)col * ldx];
-  const double* pj = part + (long)j * M;
+  const T x0 = X[(long)col * ldx];
+  const T* pj = part + (long)j * M;
   const long step = (long)ncol * M;
-  grouped_sum(S, scratch, M, nsplit, [&](int r, int i) { return pj[i * step + r]; });
-  for (int r = threadIdx.x; r < M; r += blockDim.x) S[r] = 2.0 * S[r] - W[(long)r * ldw] * x0;
-  __syncthreads();
-  double* c = C + (long)j * M;
-  if (nkb > 0) grouped_sum(c, scratch, nkb, nkb, [&](int r, int q) { return D[r + (long)q * nkb] * S[q]; });
-  for (int r = nkb + threadIdx.x; r < M; r += blockDim.x) c[r] = alpha * S[r];
+  T* cj = C + (long)j * M;
+  if constexpr (GROUPS) {
+    __shared__ T scratch[NT];
+    int rw = 32;
+    while (rw < M && rw < NT) rw *= 2;
+    const int ng = NT / rw, g = threadIdx.x / rw, rt = threadIdx.x % rw;
+    auto group_sum = [&](T mine) {  // of row rt, in group 0
+      scratch[threadIdx.x] = mine;
+      __syncthreads();
+      T sum = 0;
+      if (g == 0)
+        for (int q = 0; q < ng; ++q) sum += scratch[q * rw + rt];
+      __syncthreads();
+      return sum;
+    };
+    for (int r0 = 0; r0 < M; r0 += rw) {
+      const int r = r0 + rt;
+      T s[8] = {};
+      if (r < M) {
+        int i = g;
+        for (; i + 7 * ng < nsplit; i += 8 * ng) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) s[q] += pj[(i + q * ng) * step + r];
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+          if (i + q * ng < nsplit) s[q] += pj[(i + q * ng) * step + r];
+      }
+      const T sum = group_sum(((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+      if (g == 0 && r < M) S[r] = T(2) * sum - W[(long)r * ldw] * x0;
+    }
+    __syncthreads();
+    for (int r0 = 0; r0 < M; r0 += rw) {
+      const int r = r0 + rt;
+      T c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+      if (r < nkb) {
+        const T* d = D + r;
+        int q = g;
+        for (; q + 3 * ng < nkb; q += 4 * ng) {
+          c0 = fma(d[(long)q * nkb], S[q], c0);
+          c1 = fma(d[(long)(q + ng) * nkb], S[q + ng], c1);
+          c2 = fma(d[(long)(q + 2 * ng) * nkb], S[q + 2 * ng], c2);
+          c3 = fma(d[(long)(q + 3 * ng) * nkb], S[q + 3 * ng], c3);
+        }
+        for (; q < nkb; q += ng) c0 = fma(d[(long)q * nkb], S[q], c0);
+      }
+      const T c = group_sum((c0 + c1) + (c2 + c3));
+      if (g == 0 && r < M) cj[r] = r < nkb ? c : alpha * S[r];
+    }
+  } else {
+    for (int r = threadIdx.x; r < M; r += NT) {
+      const T w0 = W[(long)r * ldw];
+      T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+      int i = 0;
+      for (; i + 3 < nsplit; i += 4) {
+        s0 += pj[i * step + r];
+        s1 += pj[(i + 1) * step + r];
+        s2 += pj[(i + 2) * step + r];
+        s3 += pj[(i + 3) * step + r];
+      }
+      for (; i < nsplit; ++i) s0 += pj[i * step + r];
+      S[r] = T(2) * ((s0 + s1) + (s2 + s3)) - w0 * x0;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < M; r += NT) {
+      T c = 0;
+      if (r < nkb) {
+#pragma unroll 8
+        for (int q = 0; q < nkb; ++q) c = fma(D[r + (long)q * nkb], S[q], c);
+      }
+      cj[r] = r < nkb ? c : alpha * S[r];
+    }
+  }
 }
 
+// GROUPS decides the order of the sums and follows the count's bucket (512 is one's
+// bound, see bucket_systems); the number of threads without it does not.
+template <class T>
+static void gamma_reduce_t(const T* part, int nsplit, int M, int ncol, const T* W, long ldw, const T* X, long ldx,
+                           const int* cols, const T* D, int nkb, T alpha, T* C, cudaStream_t s, const int* dn, int K,
+                           int ctas) {
+  if (ncol <= 0 || M <= 0) return;
+  auto go = [&](auto k, int nt) {
+    k<<<ncol, nt, sizeof(T) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb, alpha, C, K, ctas);
+  };
+  if (ncol <= 8 * kBucketSystems) go(k_gamma_reduce<T, 512, true>, 512);
+  else if (M <= 128) go(k_gamma_reduce<T, 128, false>, 128);
+  else go(k_gamma_reduce<T, 256, false>, 256);
+}
 void gamma_reduce(const double* part, int nsplit, int M, int ncol, const double* W, long ldw, const double* X,
                   long ldx, const int* cols, const double* D, int nkb, double alpha, double* C, cudaStream_t s,
-                  const int* dn, int K, int ctas) {
-  if (ncol <= 0 || M <= 0) return;
-  k_gamma_reduce<<<ncol, red_threads(ncol), sizeof(double) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb,
-                                                        alpha, C, K, ctas);
+                  const int* dn, int K) {
+  gamma_reduce_t<double>(part, nsplit, M, ncol, W, ldw, X, ldx, cols, D, nkb, alpha, C, s, dn, K, 0);
+}
+void gamma_reduce32(const float* part, int nsplit, int M, int ncol, const float* W, long ldw, const float* X, long ldx,
+                    const int* cols, const float* D, int nkb, float alpha, float* C, cudaStream_t s, const int* dn,
+                    int K, int umma_ctas) {
+  gamma_reduce_t<float>(part, nsplit, M, ncol, W, ldw, X, ldx, cols, D, nkb, alpha, C, s, dn, K, umma_ctas);
 }
 
 // ---------------------------------------------------------------------------
@@ -326,7 +355,7 @@ constexpr int NN_STAGE = NN_R * NN_WLD + 32 * NN_CLD;
 __global__ void __launch_bounds__(128, 3) k_gemm_nn(const double* __restrict__ W, long ldw, int M,
                                                  const double* __restrict__ C, double* __restrict__ Y, long ldy,
                                                  const int* __restrict__ cols, int ncol_host, const int* dn, int K,
-                                                 double beta, int al16) {
+                                                 double beta) {
   extern __shared__ __align__(16) double nn_sm[];
   const int ncol = dev_count(dn, ncol_host);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -341,7 +370,7 @@ __global__ void __launch_bounds__(128, 3) k_gemm_nn(const double* __restrict__ W
     for (int i = 0; i < NN_R / 2; ++i) {
       const int rr = (tid >> 6) + 2 * i, r = rb + rr;
       const bool ok = r < M && k < K;
-      cp_pair(sw + rr * NN_WLD + kp, W + (ok ? (long)r * ldw + k : 0), ok, al16 != 0);
+      cp_pair(sw + rr * NN_WLD + kp, W + (ok ? (long)r * ldw + k : 0), ok);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -414,24 +443,18 @@ __global__ void __launch_bounds__(128, 3) k_gemm_nn(const double* __restrict__ W
 void gemm_nn(const double* W, long ldw, int M, const double* C, double* Y, long ldy, const int* cols, int ncol,
              int K, double beta, cudaStream_t s, const int* dn) {
   if (ncol <= 0 || M <= 0) return;
-  const int al16 = ldw % 2 == 0 && (uintptr_t)W % 16 == 0;
   constexpr int SM = (int)sizeof(double) * NN_STAGE * NN_ST;
   dim3 grid((K + 127) / 128, (ncol + 31) / 32);
-  k_gemm_nn<<<grid, 128, SM, s>>>(W, ldw, M, C, Y, ldy, cols, ncol, dn, K, beta, al16);
+  k_gemm_nn<<<grid, 128, SM, s>>>(W, ldw, M, C, Y, ldy, cols, ncol, dn, K, beta);
 }
 
 void la_setup() {
-  cudaFuncSetAttribute(k_gemm_tn<32, 32, 1, 1, 4, 64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       TnTile<32, 32, 1, 1, 4, 64, 3>::SMEM);
-  cudaFuncSetAttribute(k_gemm_tn<64, 64, 2, 2, 1, 16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       TnTile<64, 64, 2, 2, 1, 16, 4>::SMEM);
-  cudaFuncSetAttribute(k_gemm_tn<112, 64, 1, 4, 1, 16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       TnTile<112, 64, 1, 4, 1, 16, 3>::SMEM);
+  cudaFuncSetAttribute(k_gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, TN_SMEM);
   cudaFuncSetAttribute(k_gemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(double) * NN_STAGE * NN_ST);
   // S of all projectors beside the kernel's static scratch, which together pass the
   // 48 KB that a launch has without this: up to 6,144 projectors
-  cudaFuncSetAttribute(k_gamma_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+  cudaFuncSetAttribute(k_gamma_reduce<double, 512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
 }
 
 // ---------------------------------------------------------------------------
@@ -1113,41 +1136,6 @@ void gemm_tn32(const float* W, long ldw, int M, const float* X, long ldx, const 
   kchunk = (kchunk + 15) / 16 * 16;
   dim3 grid((M + 63) / 64, (ncol + 63) / 64, nsplit);
   k_gemm_tn_f32<<<grid, 256, 0, s>>>(W, ldw, M, X, ldx, cols, ncol, dn, K, kchunk, part);
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_gamma_reduce32(const float* __restrict__ part, int nsplit, int M,
-                                                        int ncol_host, const int* dn,
-                                                        const float* __restrict__ W, long ldw,
-                                                        const float* __restrict__ X, long ldx,
-                                                        const int* __restrict__ cols, const float* __restrict__ D,
-                                                        int nkb, float alpha, float* __restrict__ C, int K,
-                                                        int umma_ctas) {
-  extern __shared__ float Sf[];
-  __shared__ float scratch[kRedThreads];
-  const int ncol = dev_count(dn, ncol_host);
-  const int j = blockIdx.x;
-  if (j >= ncol) return;
-  if (dn && umma_ctas > 0) {  // the split plan of the tcgen05 bra-ket for this column count
-    int per;
-    umma_braket_plan(ncol, K, &nsplit, &per, umma_ctas);
-  }
-  const int col = cols ? cols[j] : j;
-  const float x0 = X[(long)col * ldx];
-  const float* pj = part + (long)j * M;
-  const long step = (long)ncol * M;
-  grouped_sum(Sf, scratch, M, nsplit, [&](int r, int i) { return pj[i * step + r]; });
-  for (int r = threadIdx.x; r < M; r += blockDim.x) Sf[r] = 2.f * Sf[r] - W[(long)r * ldw] * x0;
-  __syncthreads();
-  float* c = C + (long)j * M;
-  if (nkb > 0) grouped_sum(c, scratch, nkb, nkb, [&](int r, int q) { return D[r + (long)q * nkb] * Sf[q]; });
-  for (int r = nkb + threadIdx.x; r < M; r += blockDim.x) c[r] = alpha * Sf[r];
-}
-void gamma_reduce32(const float* part, int nsplit, int M, int ncol, const float* W, long ldw, const float* X, long ldx,
-                    const int* cols, const float* D, int nkb, float alpha, float* C, cudaStream_t s, const int* dn,
-                    int K, int umma_ctas) {
-  if (ncol <= 0 || M <= 0) return;
-  k_gamma_reduce32<<<ncol, red_threads(ncol), sizeof(float) * M, s>>>(part, nsplit, M, ncol, dn, W, ldw, X, ldx, cols, D, nkb, alpha,
-                                                        C, K, umma_ctas);
 }
 
 // Y[col j][k] += sum_r W[r][k] C[j][r]; tile 128 k x 32 j, r step 16
