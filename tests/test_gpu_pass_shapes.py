@@ -81,7 +81,7 @@ def _step_cell(L, ecut, nr, lo, hi):
 
 
 @pytest.mark.parametrize("form", ["fp64", "mixed"])
-@pytest.mark.parametrize("m", [2, 23])                          # 6 systems, and 69: 1,024 threads in the last cell
+@pytest.mark.parametrize("m", [2, 23])                          # 6 systems, and 69: in the last cell 1,024 threads (FP64), 512 (mixed)
 @pytest.mark.parametrize("cell", _STEP_CELLS)
 def test_step_shapes(cell, m, form):
     _check(_step_cell(*cell), m, form)

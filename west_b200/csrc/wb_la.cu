@@ -888,21 +888,26 @@ __global__ void __launch_bounds__(NT) k_cg_step(const int* act, const int* dn, i
 //     plane waves) 24 systems FP64 12.8 with 4 CTAs, 16.9 with 2, 19.9 with 1; 64
 //     systems 17.0, 16.9 and 20.8 (4 CTAs of 1024 threads 25.6: two waves).  Below
 //     4,096 plane waves one CTA: 2,400 plane waves, 64 systems 8.8, with 4 CTAs 10.8.
-//   more systems, 1024 threads, one CTA per SM: the fewest CTAs per system with which
-//     the systems in flight keep their four vectors in 96 MB of L2 between the passes.
-//     2,048 systems FP64: 8,440 plane waves 437 with 1 CTA, 571 with 2; 16,900 1,085,
-//     1,010 with 2, 1,325 with 4; 37,387 2,506, 2,649 and 2,396 with 4.  FP32: 16,900 566
-//     with 1 and 642 with 2, 37,387 1,583 with 1, 1,373 with 2 and 1,604 with 4.
+//   more systems, one CTA each, while the systems in flight keep their four vectors in
+//     L2 between the passes: two CTAs of 512 threads per SM up to 80 MB of vectors (256
+//     systems FP64: 2,400 plane waves 12.9, one CTA of 1024 threads 17.0; 4,000 18.9 and
+//     21.4; FP32: 5,200 16.9 and 21.0, 8,440 25.1 and 27.2, 10,500 38.2 and 39.4, but 1,024
+//     systems of 8,440 150 and 143, of 10,500 206 and 174), then one of 1,024.
+//   then the fewest CTAs per system with which one CTA per SM keeps to 96 MB.  2,048
+//     systems FP64: 8,440 plane waves 437 with 1 CTA, 571 with 2; 16,900 1,085, 1,010 with
+//     2, 1,325 with 4; 37,387 2,506, 2,649 and 2,396 with 4.  FP32: 16,900 566 with 1 and
+//     642 with 2, 37,387 1,583 with 1, 1,373 with 2 and 1,604 with 4.
 struct CgShape {
   int threads, ctas;
 };
 static CgShape cg_shape(int n, int npw, int elem) {
   if (npw <= 1024) return {256, 1};
-  if (npw < 4096) return {512, 1};
   const int systems = bucket_systems(n);
-  if (systems <= kBucketSystems) return {512, 4};
+  if (systems <= kBucketSystems && npw >= 4096) return {512, 4};
+  const double vectors = 4.0 * elem * npw;
+  if (vectors * 2 * sm_count() <= 80e6) return {512, 1};
   int cs = 1;
-  while (cs < 8 && 4.0 * elem * npw * (double)std::min(systems, sm_count() / cs) > 96e6) cs *= 2;
+  while (cs < 8 && vectors * std::min(systems, sm_count() / cs) > 96e6) cs *= 2;
   return {1024, cs};
 }
 template <class C, int NT, int CS, class... A>
