@@ -13,16 +13,15 @@
 namespace wb {
 
 int sm_count() {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) !=
-                                                  cudaSuccess || nsm <= 0)
-      nsm = 148;
-  }
+  static const int nsm = [] {  // contexts of several threads may ask first
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+    return n;
+  }();
   return nsm;
 }
-
 
 WB_DEV void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
