@@ -301,7 +301,6 @@ int ensure_workspace(wb_ctx* c, int mb, long ld_in, long ld_out) {
   bad |= c->items.ensure(sizeof(int2) * (nsys / 2 + 1)) != 0;
   bad |= c->nact.ensure(sizeof(int) * 4) != 0;
   bad |= c->ecol.ensure(sizeof(double) * nsys) != 0;
-  bad |= c->epcol.ensure(sizeof(double) * nsys) != 0;
   bad |= c->unconv.ensure(sizeof(int) * mb) != 0;
   bad |= c->items_pp.ensure(sizeof(int2) * mp) != 0;
   bad |= c->items_pk.ensure(sizeof(int2) * (size_t)mb * c->npv) != 0;
@@ -833,9 +832,8 @@ int run_batch(wb_ctx* c, int mb, const double2* dvg, long ld_in, double2* dng, l
   double2* T = c->T.as<double2>();
   double2* stk = c->sticks.as<double2>();
   {
-    Stage g(c, WB_STAGE_OTHER, 3, mb);
+    Stage g(c, WB_STAGE_OTHER, 2, mb);
     fill_columns(c->et.as<double>(), nocc, nsys, c->ecol.as<double>(), s);
-    fill_columns(c->eprec.as<double>(), nocc, nsys, c->epcol.as<double>(), s);
     // 1. aux = sqvc * dvg in internal order            (apply_operator.f90:49-53)
     permute_scale(dvg, ld_in, c->perm.as<int>(), c->sqvc.as<double>(), npw, mb, aux, ld, s);
   }
@@ -1239,7 +1237,7 @@ int wb_ctx_destroy(wb_ctx* c) {
   DBuf* bufs[] = {&c->perm, &c->gqz, &c->spg, &c->stpos, &c->cmap, &c->zlo, &c->zmap, &c->tw, &c->g2kin, &c->sqvc, &c->vs, &c->evc, &c->W,
                   &c->D, &c->eprec, &c->et, &c->occ, &c->evcr, &c->iprec, &c->dvg_in, &c->dng_out, &c->aux, &c->dvbox, &c->B,
                   &c->X, &c->G, &c->T, &c->sticks, &c->sticks2, &c->acc, &c->part, &c->C, &c->rho, &c->conv,
-                  &c->act, &c->items, &c->nact, &c->ecol, &c->epcol, &c->unconv, &c->items_pp, &c->items_pk,
+                  &c->act, &c->items, &c->nact, &c->ecol, &c->unconv, &c->items_pp, &c->items_pk,
                   &c->iota_items, &c->fcoef, &c->rt_colx, &c->twx, &c->twy, &c->twz, &c->twx32, &c->twy32, &c->twz32, &c->dav_dvg, &c->dav_dng, &c->dav_tmp, &c->dav_hr, &c->dav_vr, &c->dav_A,
                   &c->dav_V, &c->dav_w, &c->dav_part, &c->dav_coef, &c->dav_dots, &c->dav_bj, &c->dav_st, &c->W32, &c->D32, &c->g2kin32,
                   &c->vs32, &c->tw32, &c->g32, &c->P32, &c->T32, &c->d32, &c->sticks32, &c->part32, &c->C32,
@@ -1415,7 +1413,7 @@ struct Carve {
 struct NoallocWs {
   FftArgs fa;  // the context's, or with its sticks unpadded
   double2 *aux, *dvbox, *B, *X, *G, *T, *sticks, *sticks2, *acc;
-  double *part, *C, *rho, *ecol, *epcol;
+  double *part, *C, *rho, *ecol;
   unsigned char* conv;
   int *act, *nact, *unconv;
   int2 *items, *items_pp, *items_pk;
@@ -1454,7 +1452,6 @@ void noalloc_layout(const wb_ctx* c, int mb, int level, Carve& cv, NoallocWs& w)
   w.C = cv.take<double>(nsys * c->nproj);
   w.rho = cv.take<double>(nsys);
   w.ecol = cv.take<double>(nsys);
-  w.epcol = cv.take<double>(nsys);
   w.conv = cv.take<unsigned char>(nsys);
   w.act = cv.take<int>(nsys);
   w.nact = cv.take<int>(4);
@@ -1511,7 +1508,6 @@ int noalloc_run(wb_ctx* c, const NoallocWs& w, int mb, const double2* dvg, long 
   const int nit = std::max(mp, mb * npv);
   k_noalloc_items<<<(nit + 255) / 256, 256, 0, s>>>(w.items_pp, w.items_pk, mb, nocc, npv);
   fill_columns(c->et.as<double>(), nocc, nsys, w.ecol, s);
-  fill_columns(c->eprec.as<double>(), nocc, nsys, w.epcol, s);
   permute_scale(dvg, ld_in, c->perm.as<int>(), c->sqvc.as<double>(), npw, mb, w.aux, ld, s);
   fft_zinv(w.fa, w.aux, ld, w.items_pp, mp, w.sticks);
   fft_plane_inv_box(w.fa, w.sticks, mp, w.dvbox);

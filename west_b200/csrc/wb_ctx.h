@@ -69,7 +69,7 @@ struct wb_ctx {
   DBuf perm, gqz, spg, stpos, cmap, zlo, zmap, tw, g2kin, sqvc, vs, evc, W, D, eprec, et, occ, evcr, iprec;
   // per-call workspace
   DBuf dvg_in, dng_out, aux, dvbox, B, X, G, T, sticks, sticks2, acc, part, C, rho, conv, act, items, nact,
-      ecol, epcol, unconv, items_pp, items_pk, iota_items, fcoef;
+      ecol, unconv, items_pp, items_pk, iota_items, fcoef;
   int* nact_host = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   wb_stats stats{};

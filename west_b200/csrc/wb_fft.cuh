@@ -31,7 +31,6 @@ template <> struct FftSplit<80> { static constexpr int N1 = 8, N2 = 10; };
 template <> struct FftSplit<96> { static constexpr int N1 = 8, N2 = 12; };
 template <> struct FftSplit<100> { static constexpr int N1 = 10, N2 = 10; };
 template <> struct FftSplit<108> { static constexpr int N1 = 12, N2 = 9; };
-template <> struct FftSplit<120> { static constexpr int N1 = 12, N2 = 10; };
 
 // Literal constants of the radix-3 and radix-5 butterflies.
 constexpr double kS3 = 0.86602540378443864676;   // sin(2 pi / 3)
@@ -43,7 +42,7 @@ constexpr double kS52 = 0.58778525229247312917;  // sin(4 pi / 5)
 constexpr double kC71 = 0.62348980185873353053, kC72 = -0.22252093395631440429, kC73 = -0.90096886790241912624;
 constexpr double kS71 = 0.78183148246802980871, kS72 = 0.97492791218182360702, kS73 = 0.43388373911755812048;
 
-// Composite radices R = A * B of the register DFT.  6, 10, 12, 14 and 15 have
+// Composite radices R = A * B of the register DFT.  6, 10, 12 and 15 have
 // coprime factors and run the prime-factor map (no inner twiddles); 8, 9 and 16
 // take theirs from literals.
 template <int R> struct Factor2;
@@ -52,10 +51,9 @@ template <> struct Factor2<8> { static constexpr int A = 4, B = 2; };
 template <> struct Factor2<9> { static constexpr int A = 3, B = 3; };
 template <> struct Factor2<10> { static constexpr int A = 5, B = 2; };
 template <> struct Factor2<12> { static constexpr int A = 4, B = 3; };
-template <> struct Factor2<14> { static constexpr int A = 7, B = 2; };
 template <> struct Factor2<15> { static constexpr int A = 5, B = 3; };
 template <> struct Factor2<16> { static constexpr int A = 4, B = 4; };
-constexpr bool pfa_radix(int r) { return r == 6 || r == 10 || r == 12 || r == 14 || r == 15; }
+constexpr bool pfa_radix(int r) { return r == 6 || r == 10 || r == 12 || r == 15; }
 // the inverse of x modulo m (x, m coprime, small)
 constexpr int inv_mod(int x, int m) {
   for (int i = 1; i < m; ++i)
