@@ -12,7 +12,7 @@ import json
 import os
 import sys
 
-ref = sys.argv[1] if len(sys.argv) > 1 else "/root/reference"
+ref = sys.argv[1]
 w = json.load(open(os.path.join(ref, "test-suite/test001/ref/wstat.json")))
 par = json.load(open(os.path.join(ref, "test-suite/parameters.json")))
 ctl = w["input"]["wstat_control"]

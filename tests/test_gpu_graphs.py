@@ -2,10 +2,9 @@
 tested on the device by a conditional WHILE node) against the eager loops
 (host readback of the active count every iteration) and the FP64 oracle.
 
-The two paths run the same kernels; the graph path sizes grids for the
-workspace capacity and strides over the active systems, and its split-K
-GEMMs may use a different split count, so FP64 results agree to rounding
-(1e-12) and the iteration counts agree exactly."""
+The two paths run the same kernels with the same order of sums (the graph
+path sizes grids for the workspace capacity); FP64 results agree to 1e-12 and the
+iteration counts exactly."""
 import numpy as np
 import pytest
 
