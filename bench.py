@@ -363,6 +363,10 @@ def run_b200(args, rank, world, local_rank):
                          "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": traffic, "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback",
                          "algorithmic_bytes_per_launch": per_launch_bytes,
+                         "note": "achieved counts the dense-box model's bytes (2 box FFTs per item), of which the "
+                                 "stick decomposition moves a fifth: frac may pass 1 and is no share of the HBM "
+                                 "rate; dram_frac is that, from the profiled traffic (profiles/)",
+                         "dram_frac": traffic / per_launch_s / 1e9 / hbm if traffic else None,
                          "fp64": {"achieved_tflops_nominal": fp64_ach, "dgemm_peak_tflops": fp64_peak,
                                   "frac": fp64_ach / fp64_peak}},
             "stage_share": stage_share,
