@@ -52,8 +52,8 @@ WB_DEV void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "
 // (4 rows x 4 k) on distinct banks.  K is even and a stage reads pairs of k.
 // One tile for every size.  Bound by the FP64 tensor pipe (36.9 TFLOP/s) and its own
 // latency.  Against two larger ones with a warp per k, us and TFLOP/s: 64 rows, 2,048
-// columns, K = 16,880 154 and 29 (64 x 64: 142); 112 rows, 384 columns, K = 33,800 114
-// and 25 (112 x 64: 97), 208 rows, 384 columns, K = 74,774 413 and 29 (112 x 64: 416); but
+// columns, K = 16,880 152 and 29 (64 x 64: 142); 112 rows, 384 columns, K = 33,800 111
+// and 26 (112 x 64: 97), 208 rows, 384 columns, K = 74,774 411 and 29 (112 x 64: 416); but
 // 80 rows, 256 columns, K = 4,800 15 (112 x 64: 34), 32 rows, 2,048 columns, K = 16,880 83
 // (64 x 64: 140).  Their chains of additions are four times as long: error against sums
 // in extended precision 1.4e-15 and 1.9e-15 at the first and third size, here 5.2e-16
