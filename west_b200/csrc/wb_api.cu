@@ -369,10 +369,11 @@ int autotune32(wb_ctx* c, int nsys) {
 }
 
 // A branch of the pass being captured on the context's second stream, and its
-// end.  It pays while a pass is launch and chain latency (one perturbation at
-// 64^3: 5.0 -> 4.7 ms a call, at 24^3 0.86 -> 0.75); with hundreds of systems
-// every kernel fills the GPU and the two branches only share its L2 (108^3, 512
-// systems: 276 against 284 ms).
+// end.  It pays while a pass is launch and chain latency; with many systems every
+// kernel fills the GPU and the branches share its L2.  Decided per bucket.  Calls with
+// the branch in every bucket over calls without it: one perturbation 0.81 at 48^3, 0.83
+// at 64^3, 0.89 at 80^3, 0.96 at 108^3; 2 to 5 million systems x plane waves 0.94 to 1.00;
+// 64^3, 9 million 1.00 (mixed 1.01) and 17 million 1.01.
 bool forked(const wb_ctx* c, int nmax) { return (double)nmax * c->npw <= 8e6; }
 cudaStream_t fork_side(wb_ctx* c) {
   cudaEventRecord(c->side_ev[0], c->stream);
