@@ -1578,8 +1578,8 @@ extern "C" int wb_apply_operator_device_noalloc(wb_ctx* c, int m, const double* 
     return fail(WB_ERR_ARG, "m = " + std::to_string(m) + " perturbations do not fit the allocation-free entry "
                 "point's scratch of " + std::to_string((size_t)WB_NOALLOC_SCRATCH_BYTES) +
                 " bytes (WB_NOALLOC_SCRATCH_BYTES): use fewer perturbations per call");
-  // the first level that fits: with the split plan of the other entry points, up to
-  // 64 systems give their bits; unpadded sticks keep the largest calls within the
+  // the first level that fits: with the split plan of the other entry points a call
+  // gives their bits; unpadded sticks keep the largest calls within the
   // scratch (75 perturbations of 7 bands at 24^3: 32.9 MB of 33.6, padded 34.2)
   Carve probe{nullptr};
   NoallocWs w{};
